@@ -6,6 +6,7 @@
 #include <cooperative_groups.h>
 
 #include "abd_common.cuh"
+#include "abd_merge.cuh"
 
 namespace abd {
 namespace precond {
@@ -309,6 +310,16 @@ __device__ inline long long block_scan_excl(long long v, long long* total) {
   return before;
 }
 
+// a CTA of KT threads, for merge_rounds
+template <int KT>
+struct CtaTeam {
+  __device__ __forceinline__ int id() const { return (int)threadIdx.x; }
+  __device__ __forceinline__ int size() const { return KT; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+  __device__ __forceinline__ bool any(bool p) const { return __syncthreads_or(p) != 0; }
+  __device__ __forceinline__ void best(unsigned long long* p, unsigned long long key) const { atomicMax(p, key); }
+};
+
 // The preconditioner's clusters, formed on the device by one CTA from the active-pair list
 // the pair assembly appended (pair, I, J, FP32 weight bits; in any order).  Rounds: every
 // cluster picks its strongest admissible pair to another cluster (weight, then the lower pair
@@ -327,42 +338,10 @@ __device__ void make_clusters(int n, int cap, const int4* act, int cap_act, cons
     w.label[b] = b;
     w.size[b] = 1;
   }
-  __shared__ int merged, nsolo, nmulti;
+  __shared__ int nsolo, nmulti;
   if (tid == 0) nsolo = nmulti = 0;
   __syncthreads();
-  for (int round = 0; cap > 1 && round < 4 * kMaxCluster; ++round) {
-    for (int b = tid; b < n; b += KT) {
-      w.best[b] = 0ULL;
-      w.to[b] = b;
-    }
-    if (tid == 0) merged = 0;
-    __syncthreads();
-    for (int e = tid; e < m; e += KT) {
-      const int4 q = act[e];
-      const int a = w.label[q.y], b = w.label[q.z];
-      if (a == b || w.size[a] + w.size[b] > cap) continue;
-      const unsigned long long key = ((unsigned long long)(unsigned)q.w << 32) | (0xffffffffULL - (unsigned)q.x);
-      atomicMax(&w.best[a], key);
-      atomicMax(&w.best[b], key);
-    }
-    __syncthreads();
-    // a cluster has one best pair, so it takes part in at most one merge of the round
-    for (int e = tid; e < m; e += KT) {
-      const int4 q = act[e];
-      const int a = w.label[q.y], b = w.label[q.z];
-      if (a == b) continue;
-      const unsigned long long key = ((unsigned long long)(unsigned)q.w << 32) | (0xffffffffULL - (unsigned)q.x);
-      if (w.best[a] != key || w.best[b] != key) continue;
-      const int r = min(a, b), o = max(a, b);
-      w.to[o] = r;
-      w.size[r] += w.size[o];
-      merged = 1;
-    }
-    __syncthreads();
-    for (int b = tid; b < n; b += KT) w.label[b] = w.to[w.label[b]];
-    __syncthreads();
-    if (!merged) break;
-  }
+  merge_rounds(CtaTeam<KT>{}, n, cap, 4 * kMaxCluster, act, m, w);
   // cluster index of every label, cluster offsets and inverse offsets, in label order
   long long ccarry = 0, pcarry = 0, ocarry = 0;
   for (int b0 = 0; b0 < n; b0 += KT) {
