@@ -10,6 +10,7 @@
 
 #include "../../include/abd_b200.h"
 #include "abd_exact.cuh"
+#include "abd_rounds.cuh"
 
 namespace abd {
 
@@ -506,6 +507,7 @@ struct StepDev {
   int again;         // the Newton loop ended for that
   int run;           // (batches) the scene takes part in the round
   int lists;         // candidate lists made
+  int rounds;        // rounds begun
   double E0, E1;     // energy of the current iterate and of the accepted one
   double alpha, toi; // the last accepted step length and raw time of impact
   unsigned long long t0, t1;       // first start and last end (ns) of the current narrow launch

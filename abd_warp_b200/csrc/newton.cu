@@ -58,7 +58,7 @@ __global__ void k_step_begin(Mailbox* box, cudaGraphConditionalHandle h, int n, 
   StepDev& S = box->step;
   S.it = S.lin = S.ls = 0;
   S.n_pt = S.n_ee = S.n_vg = S.n_ij = S.n_active = 0;
-  S.resume = S.again = S.lists = 0;
+  S.resume = S.again = S.lists = S.rounds = 0;
   S.run = 1;
   S.E0 = S.E1 = S.alpha = 0.0;
   S.toi = 1.0;
@@ -77,15 +77,21 @@ __global__ void k_round_begin(Mailbox* box, const int* bad, int* cand, int cap_p
   const bool run = !shared || box->step.run;
   if (threadIdx.x == 0) {
     box->step.again = 0;
+    if (run) ++box->step.rounds;
     cudaGraphSetConditional(h_list, run && *bad ? 1u : 0u);
     if (!shared) cudaGraphSetConditional(h_newton, 1u);
   }
   if (run) clear_gh(ds, cand, cap_pairs, threadIdx.x, blockDim.x);
 }
 
-// A round's end: another one when an iteration left the list's region.
-__global__ void k_round_end(Mailbox* box, cudaGraphConditionalHandle h) {
-  cudaGraphSetConditional(h, box->step.again && !(box->dstat[DS_STATUS] & kRerunMask) ? 1u : 0u);
+// A round's end: another one when an iteration left the list's region (and one can be due).
+__global__ void k_round_end(Mailbox* box, int max_iter, cudaGraphConditionalHandle h) {
+  bool more = box->step.again && !(box->dstat[DS_STATUS] & kRerunMask);
+  if (more && !another_round(box->step.rounds, max_iter)) {
+    box->dstat[DS_STATUS] |= ST_LS_MORE;  // (never; the host finishes the step)
+    more = false;
+  }
+  cudaGraphSetConditional(h, more ? 1u : 0u);
 }
 
 // A Newton iteration's end.  Every CTA makes the backtracking line search's decision (abd.py:146-160)
@@ -210,7 +216,7 @@ cudaError_t round_begin(Sim& s, cudaGraphConditionalHandle h_list, cudaGraphCond
 }
 
 cudaError_t round_end(Sim& s, cudaGraphConditionalHandle h_round) {
-  k_round_end<<<1, 1, 0, s.stream>>>(s.box, h_round);
+  k_round_end<<<1, 1, 0, s.stream>>>(s.box, s.prm.max_iter, h_round);
   ++s.launches;
   return cudaGetLastError();
 }

@@ -246,10 +246,20 @@ __global__ void __launch_bounds__(LT, 2) k_newton_batch(const LoopArgs* scenes, 
   }
 }
 
-// A round's end: another one while a scene's iteration left its list's region
+// A round's end: another one while a scene's iteration left its list's region (and one can be due, as
+// in k_round_end)
 __global__ void __launch_bounds__(128) k_batch_end(const LoopArgs* scenes, int n, cudaGraphConditionalHandle h) {
   int more = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) more |= scenes[i].box->step.run;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    Mailbox* const box = scenes[i].box;
+    if (!box->step.run) continue;
+    if (another_round(box->step.rounds, scenes[i].gh.prm.max_iter)) {
+      more = 1;
+    } else {
+      box->step.run = 0;
+      box->dstat[DS_STATUS] |= ST_LS_MORE;
+    }
+  }
   more = __syncthreads_or(more);
   if (threadIdx.x == 0) cudaGraphSetConditional(h, more ? 1u : 0u);
 }
