@@ -202,10 +202,14 @@ __device__ inline int next_block(Ctx& c, int b) {
     for (int l = l##b + c.tid; l < min(c.nrow, l##b + kRowBlock); l += c.T)
 
 // The solve by a cluster of C CTAs, this one the rank-th.  dyn: the CTA's dynamic shared memory;
-// red: in shared memory
+// red: in shared memory.  NC: the kernel is the solve alone; then no barrier has told yet that every
+// CTA of the cluster runs, which the first store to another CTA's shared memory needs: each
+// arrives here and waits just before its first dot products, when the others have long arrived.
+// (Without NC the caller has passed a cluster barrier.)
 template <bool PCG, bool NC>
 __device__ __forceinline__ void solve(const KrylovArgs& a, double* dyn, RedShared& red, int C, int rank) {
   __shared__ int sh_p[2];
+  if (NC && C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   Ctx c;
   c.T = (int)blockDim.x;
   c.tid = (int)threadIdx.x;
@@ -282,6 +286,7 @@ __device__ __forceinline__ void solve(const KrylovArgs& a, double* dyn, RedShare
     S_a[l] = bi;
   }
   __syncthreads();
+  if (NC && C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   FOR_ROWS(l) {
     const double2 m = apply_rows<NC>(a, pos[l / 12], l, S_r, S_a);
     add(c, 0, S_r[l] * m.x);
