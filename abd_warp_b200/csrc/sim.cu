@@ -1689,8 +1689,10 @@ int abd_batch_step(abd_batch* b, const abd_states* st, double* const* x_view, ab
     if (r == ABD_OK && e2 != cudaSuccess) r = ABD_ERR_CUDA;
     if (r == ABD_OK && ABD_NOTE(cudaGraphInstantiate(&b->exec, graph, 0)) != cudaSuccess) r = ABD_ERR_CUDA;
     if (graph) cudaGraphDestroy(graph);
+    // (on the stream that launches the graph, which no other stream's order binds; the wait is for slots)
     if (r == ABD_OK && !slots.empty() &&
-        ABD_NOTE(cudaMemcpy(b->args, slots.data(), slots.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+        (ABD_NOTE(cudaMemcpyAsync(b->args, slots.data(), slots.size(), cudaMemcpyHostToDevice, b->stream)) != cudaSuccess ||
+         ABD_NOTE(cudaStreamSynchronize(b->stream)) != cudaSuccess))
       r = ABD_ERR_CUDA;
     if (r != ABD_OK) {
       if (b->exec) cudaGraphExecDestroy(b->exec);
