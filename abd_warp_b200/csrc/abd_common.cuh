@@ -322,12 +322,17 @@ struct Sim {
   double* reg = nullptr;
   int* ext = nullptr;              // [n][kExt] vertices extreme in fixed rest-frame directions
   double* gh_q = nullptr;          // [12 n] the DOFs (A, then p) of the device loop's last GH pass
-  // the device loop's last GH pass numbered its body pairs by the list; their exact set (the
-  // exported one) is made when abd_export_system asks for it
+  // the device loop's last GH pass numbered its body pairs by the list (and nothing has replaced that
+  // system or its pair arrays since); its exact pairs, at gh_q with the step's parameters, are made
+  // when a call asks for them (gather_system): x_n of them (-1: not made), their blocks and counts
   bool sys_list = false;
-  int2* x_ij = nullptr;            // that set [x_cap], its scratch
-  int x_cap = 0;
-  int *x_row = nullptr, *x_cnt = nullptr;  // [2 (n + 1)], [2 n]
+  double sys_dhat = 0.0;
+  int sys_friction = 0;
+  int x_n = -1, x_cap = 0;
+  int2* x_ij = nullptr;            // [x_cap]
+  double* x_off = nullptr;         // [x_cap][288], as offdiag
+  int* x_act = nullptr;            // [x_cap], as pair_active
+  int *x_row = nullptr, *x_cnt = nullptr;  // scratch: [2 (n + 1)], [2 n]
   double* q_last = nullptr;        // [12 n] the DOFs (A, then p) the last step ended with
   int* highlight = nullptr;        // [n] contact flags of the last GH pass (k_body_gh)
   // captured passes: CCD bound (with events for profiling), GH, line-search batches (step lengths from the host or from the CCD pass on the device)
@@ -582,9 +587,11 @@ cudaError_t body_broad(Sim& s, const double* A, const double* p, const double* A
 cudaError_t body_pairs(Sim& s, bool full, bool sup = false, const uint32_t* forced = nullptr, bool ccd = false);
 // the pairs, their scan and fill from body_sup as it stands (the kept list's pairs)
 cudaError_t list_pairs(Sim& s, const uint32_t* forced);
-// the exact body pairs at DOFs (A, p) into x_ij (body_box, the mask and x_row, x_cnt are its
+// the exact body pairs at gh_q (sys_list) into x_ij (body_box, the mask and x_row, x_cnt are its
 // scratch; the count in x_row[n + 1 + n])
-cudaError_t exact_pairs(Sim& s, const double* A, const double* p, const uint32_t* forced);
+cudaError_t exact_pairs(Sim& s);
+// those pairs, whose mask and x_row the last exact_pairs left, in place of the pair list and the adjacency
+cudaError_t install_pairs(Sim& s);
 // the number of exact body pairs at (A, p), added to *count (on stream st; body_bnd and body_box
 // are its scratch)
 cudaError_t count_pairs(Sim& s, const double* A, const double* p, int* count, cudaStream_t st);
@@ -614,8 +621,10 @@ cudaError_t prepare_narrow(Sim& s);  // kernel attributes (once, at creation)
 // were kept (dint[kSupHave]) and the step starts from the DOFs the last step ended with.
 cudaError_t gh_superset_check(Sim& s, const abd_states* st, int mode);
 cudaError_t vg_list(Sim& s, const double* y0);
+// blocks and pairs of the last system (sys_list: from the gathered ones)
 cudaError_t export_system(Sim& s, double* off_dev, int* ij_dev, int cap);
-cudaError_t export_list_system(Sim& s, double* off_dev, int* ij_dev, int cap);  // (sys_list)
+// the blocks and active counts of the x_ij pairs from the list's numbering into x_off, x_act
+cudaError_t gather_blocks(Sim& s, int n_pairs);
 cudaError_t update_dofs(Sim& s, const double* A, const double* p, const double* dq, double alpha, double* Aout,
                         double* pout);
 cudaError_t finish_step(Sim& s, const abd_states& st, double* xview);

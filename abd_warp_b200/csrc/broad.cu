@@ -693,24 +693,25 @@ __global__ void __launch_bounds__(128) k_count_pairs(int n, const Box* __restric
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
 }
 
-static cudaError_t exact_boxes(Sim& s, const double* A, const double* p, cudaStream_t st) {
+static cudaError_t exact_boxes(Sim& s, const double* A, const double* p, double dhat, cudaStream_t st) {
   k_body_bounds<<<blocks(32LL * s.nslice, 256), 256, 0, st>>>(s.nslice, s.slice, s.x0, A, p, s.body_bnd);
-  k_exact_boxes<<<blocks(s.n, 128), 128, 0, st>>>(s.n, s.body_bnd, 0.5 * s.prm.dhat, s.body_box);
+  k_exact_boxes<<<blocks(s.n, 128), 128, 0, st>>>(s.n, s.body_bnd, 0.5 * dhat, s.body_box);
   s.launches += 2;
   return cudaGetLastError();
 }
 
 cudaError_t count_pairs(Sim& s, const double* A, const double* p, int* count, cudaStream_t st) {
-  const cudaError_t e = exact_boxes(s, A, p, st);
+  const cudaError_t e = exact_boxes(s, A, p, s.prm.dhat, st);
   if (e != cudaSuccess) return e;
   k_count_pairs<<<s.n, 128, 0, st>>>(s.n, s.body_box, count);
   ++s.launches;
   return cudaGetLastError();
 }
 
-cudaError_t exact_pairs(Sim& s, const double* A, const double* p, const uint32_t* forced) {
-  const cudaError_t e = exact_boxes(s, A, p, s.stream);
+cudaError_t exact_pairs(Sim& s) {
+  const cudaError_t e = exact_boxes(s, s.gh_q, s.gh_q + 9 * (size_t)s.n, s.sys_dhat, s.stream);
   if (e != cudaSuccess) return e;
+  const uint32_t* forced = s.sys_friction ? s.fric_mask : nullptr;  // (the step's friction pairs)
   int *row = s.x_row, *upper = s.x_row + s.n + 1, *rcnt = s.x_cnt, *ucnt = s.x_cnt + s.n;
   k_pair_mask<<<s.n, PR_THREADS, 0, s.stream>>>(s.n, s.W, s.body_box, forced, s.pair_mask, s.pair_wpre, rcnt, ucnt,
                                                 s.nbr);
@@ -718,6 +719,19 @@ cudaError_t exact_pairs(Sim& s, const double* A, const double* p, const uint32_t
   k_pair_fill<<<blocks((long long)s.n * s.W, 256), 256, 0, s.stream>>>(s.n, s.W, s.pair_mask, s.pair_wpre, row, upper,
                                                                       s.x_cap, 0, s.x_ij, nullptr, nullptr);
   s.launches += 3;
+  return cudaGetLastError();
+}
+
+cudaError_t install_pairs(Sim& s) {
+  cudaError_t e = cudaMemcpyAsync(s.row_ptr, s.x_row, sizeof(int) * (s.n + 1), cudaMemcpyDeviceToDevice, s.stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(s.upper_ptr, s.x_row + s.n + 1, sizeof(int) * (s.n + 1), cudaMemcpyDeviceToDevice, s.stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(s.dint + kListBad, 1, sizeof(int), s.stream);  // (not 0: renumbered)
+  if (e != cudaSuccess) return e;
+  k_pair_fill<<<blocks((long long)s.n * s.W, 256), 256, 0, s.stream>>>(s.n, s.W, s.pair_mask, s.pair_wpre, s.row_ptr,
+                                                                      s.upper_ptr, s.cap_pairs, s.cap_adj, s.ij,
+                                                                      s.adj_col, s.adj_pair);
+  ++s.launches;
   return cudaGetLastError();
 }
 

@@ -19,6 +19,7 @@
 // vertex-ground terms (vg_ipc.py:4-34, culling.py:54-82, ccd.py:9-18, energy.py:24-33).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 
 #include "abd_graph.cuh"
@@ -1296,14 +1297,13 @@ cudaError_t vg_list_swept(Sim& s, const double* y0, const double* y1) {
   return cudaGetLastError();
 }
 
-// the same for a system numbered by the kept list's pairs: pair q of the exact set is looked up in
-// the adjacency (row I lists its neighbours in increasing order); a pair that only an exact box
-// test lists has no contact, so no block
-__global__ void k_export_list(int np, const int2* x_ij, const int* row_ptr, const int* adj_col, const int* adj_pair,
-                              const int* pair_active, const int* fixed, const double* offdiag, double* out, int* ijout,
-                              int cap) {
+// Pair q of the exact set x_ij in a system numbered by the kept list's pairs, looked up in the adjacency
+// (row I lists its neighbours in increasing order): its blocks and active contacts (none when it is
+// not listed: the list holds every pair that has a contact)
+__global__ void __launch_bounds__(128) k_gather_blocks(const int2* x_ij, const int* row_ptr, const int* adj_col,
+                                                       const int* adj_pair, const int* pair_active,
+                                                       const double* offdiag, double* x_off, int* x_act) {
   const int q = blockIdx.x;
-  if (q >= np || q >= cap) return;
   const int2 ij = x_ij[q];
   int pr = -1;
   for (int lo = row_ptr[ij.x], hi = row_ptr[ij.x + 1] - 1; lo <= hi && pr < 0;) {
@@ -1312,27 +1312,26 @@ __global__ void k_export_list(int np, const int2* x_ij, const int* row_ptr, cons
     else if (col < ij.y) lo = mid + 1;
     else hi = mid - 1;
   }
-  const bool live = pr >= 0 && pair_active[pr] > 0 && !fixed[ij.x] && !fixed[ij.y];
-  for (int e = threadIdx.x; e < 144; e += blockDim.x) out[(size_t)q * 144 + e] = live ? offdiag[(size_t)pr * 288 + e] : 0.0;
-  if (threadIdx.x == 0 && ijout) {
-    ijout[2 * q] = ij.x;
-    ijout[2 * q + 1] = ij.y;
-  }
+  const bool live = pr >= 0 && pair_active[pr] > 0;
+  for (int e = threadIdx.x; e < 288; e += blockDim.x) x_off[(size_t)q * 288 + e] = live ? offdiag[(size_t)pr * 288 + e] : 0.0;
+  if (threadIdx.x == 0) x_act[q] = live ? pair_active[pr] : 0;
 }
 
-cudaError_t export_list_system(Sim& s, double* off_dev, int* ij_dev, int cap) {
-  const int np = s.n_pairs < cap ? s.n_pairs : cap;
-  if (np == 0) return cudaSuccess;
-  k_export_list<<<np, 128, 0, s.stream>>>(s.n_pairs, s.x_ij, s.row_ptr, s.adj_col, s.adj_pair, s.pair_active, s.fixed,
-                                          s.offdiag, off_dev, ij_dev, cap);
+cudaError_t gather_blocks(Sim& s, int n_pairs) {
+  if (n_pairs == 0) return cudaSuccess;
+  k_gather_blocks<<<n_pairs, 128, 0, s.stream>>>(s.x_ij, s.row_ptr, s.adj_col, s.adj_pair, s.pair_active, s.offdiag,
+                                                 s.x_off, s.x_act);
   ++s.launches;
   return cudaGetLastError();
 }
 
 cudaError_t export_system(Sim& s, double* off_dev, int* ij_dev, int cap) {
-  const int np = s.n_pairs < cap ? s.n_pairs : cap;
-  if (np == 0) return cudaSuccess;
-  k_export_off<<<np, 128, 0, s.stream>>>(s.n_pairs, s.pair_active, s.fixed, s.offdiag, s.ij, off_dev, ij_dev, cap);
+  const int have = s.sys_list ? s.x_n : std::min(s.n_pairs, s.cap_pairs), np = std::min(have, cap);
+  if (np <= 0) return cudaSuccess;
+  if (s.sys_list)
+    k_export_off<<<np, 128, 0, s.stream>>>(np, s.x_act, s.fixed, s.x_off, s.x_ij, off_dev, ij_dev, cap);
+  else
+    k_export_off<<<np, 128, 0, s.stream>>>(np, s.pair_active, s.fixed, s.offdiag, s.ij, off_dev, ij_dev, cap);
   ++s.launches;
   return cudaGetLastError();
 }

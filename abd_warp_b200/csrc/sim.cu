@@ -937,7 +937,7 @@ int abd_sim_destroy(abd_sim* h) {
                   s.cl_tab, s.cl_inv, s.pair_wpre, s.act_pairs, s.chunk,
                   s.red_count, s.body_bnd, s.contacts, s.contacts_by_pair, s.ccd_cand, s.ecand, s.body_rest,
                   s.body_sup, s.slice, s.q_last, s.highlight, s.cl_work_buf, s.dq_save, s.adj_x,
-                  s.chunk_act, s.fric, s.fric_mask, s.list, s.reg, s.ext, s.gh_q, s.x_ij, s.x_row, s.x_cnt};
+                  s.chunk_act, s.fric, s.fric_mask, s.list, s.reg, s.ext, s.gh_q, s.x_ij, s.x_off, s.x_act, s.x_row, s.x_cnt};
   for (void* q : bufs)
     if (q) cudaFree(q);
   for (abd::GraphSlot* g : {&s.g_ccd, &s.g_ccd_ev, &s.g_gh, &s.g_gh0, &s.g_ls, &s.g_ls_dev, &s.g_step})
@@ -1053,11 +1053,53 @@ int abd_update_mesh_vertex(abd_sim* h, const double* A, const double* p, double*
 
 namespace {
 
+// The exact pairs of a device-loop step's last system (sys_list), with their blocks, into x_*
+int gather_system(Sim& s) {
+  if (s.x_n >= 0) return ABD_OK;
+  for (int tries = 0; tries < 2; ++tries) {
+    CK(abd::exact_pairs(s));
+    CK(cudaMemcpyAsync(s.hstat + 22, s.x_row + 2 * (size_t)s.n + 1, sizeof(int), cudaMemcpyDeviceToHost, s.stream));
+    CK(cudaStreamSynchronize(s.stream));
+    const int np = s.hstat[22];
+    if (np <= s.x_cap) {
+      CK(abd::gather_blocks(s, np));
+      s.x_n = np;
+      return ABD_OK;
+    }
+    for (void* q : {(void*)s.x_ij, (void*)s.x_off, (void*)s.x_act})
+      if (q) cudaFree(q);
+    s.x_ij = nullptr;
+    s.x_off = nullptr;
+    s.x_act = nullptr;
+    s.x_cap = 0;
+    if (dalloc(&s.x_ij, np) || dalloc(&s.x_off, 288 * (size_t)np) || dalloc(&s.x_act, np)) return ABD_ERR_OVERFLOW;
+    s.x_cap = np;
+  }
+  return ABD_ERR_DEVICE;
+}
+
+// The device loop's last system as a GH pass of its own leaves one, its pairs the exact ones, before
+// a pass that replaces the pair list and the adjacency
+int settle_system(Sim& s) {
+  if (!s.sys_list) return ABD_OK;
+  s.x_n = -1;  // (install_pairs needs the mask that exact_pairs leaves)
+  if (int r = gather_system(s)) return r;
+  const int np = std::min(s.x_n, s.cap_pairs);
+  CK(abd::install_pairs(s));
+  CK(cudaMemcpyAsync(s.offdiag, s.x_off, sizeof(double) * 288 * (size_t)np, cudaMemcpyDeviceToDevice, s.stream));
+  CK(cudaMemcpyAsync(s.pair_active, s.x_act, sizeof(int) * (size_t)np, cudaMemcpyDeviceToDevice, s.stream));
+  s.n_pairs = np;
+  s.n_adj = 2 * np;
+  s.sys_list = false;
+  return ABD_OK;
+}
+
 // lists (culling in LISTS mode) plus the VG list; counts = {pairs, PT, EE, VG}
 int cull_lists(abd_sim* h, const double* A, const double* p, const double* A1, const double* p1, double* y0,
                double* y1, int counts[4]) {
   Sim& s = h->s;
   const abd::Dofs d0 = direct(A, p), d1 = direct(A1, p1);
+  if (int r = settle_system(s)) return r;
   for (int tries = 0;; ++tries) {
     int r = culling(h, A ? &d0 : nullptr, A && A1 ? &d1 : nullptr, y0, y1, abd::NARROW_LISTS);
     if (r) return r;
@@ -1078,24 +1120,6 @@ int cull_lists(abd_sim* h, const double* A, const double* p, const double* A1, c
 }  // namespace
 
 extern "C" {
-
-// The body pairs of a device-loop step's last GH pass (whose contacts are numbered by the kept
-// list's pairs): the exact set at that pass's DOFs, for the export
-static int exact_system_pairs(Sim& s) {
-  const uint32_t* forced = s.prm.friction_mu > 0.0 ? s.fric_mask : nullptr;
-  for (int tries = 0; tries < 2; ++tries) {
-    CK(abd::exact_pairs(s, s.gh_q, s.gh_q + 9 * (size_t)s.n, forced));
-    CK(cudaMemcpyAsync(s.hstat + 22, s.x_row + 2 * (size_t)s.n + 1, sizeof(int), cudaMemcpyDeviceToHost, s.stream));
-    CK(cudaStreamSynchronize(s.stream));
-    s.n_pairs = s.hstat[22];
-    if (s.n_pairs <= s.x_cap) return ABD_OK;
-    if (s.x_ij) cudaFree(s.x_ij);
-    s.x_ij = nullptr;
-    s.x_cap = s.n_pairs;
-    if (dalloc(&s.x_ij, s.x_cap)) return ABD_ERR_OVERFLOW;
-  }
-  return ABD_OK;
-}
 
 int abd_collision_set(abd_sim* h, const double* y0, const double* y1, int counts[4]) {
   if (!h || !y0 || !counts) return ABD_ERR_INVALID;
@@ -1131,13 +1155,13 @@ int abd_ipc_gh(abd_sim* h, const abd_states* st, const double* A, const double* 
 int abd_export_system(abd_sim* h, double* g, double* diag, double* off, int* ij, int cap, int* n_pairs) {
   if (!h) return ABD_ERR_INVALID;
   Sim& s = h->s;
-  if (s.sys_list && s.n_pairs < 0)
-    if (int r = exact_system_pairs(s)) return r;
+  if (s.sys_list)
+    if (int r = gather_system(s)) return r;
   if (g) CK(cudaMemcpyAsync(g, s.g, sizeof(double) * 12 * s.n, cudaMemcpyDeviceToDevice, s.stream));
   if (diag) CK(cudaMemcpyAsync(diag, s.diag, sizeof(double) * 144 * s.n, cudaMemcpyDeviceToDevice, s.stream));
-  if (off) CK(s.sys_list ? abd::export_list_system(s, off, ij, cap) : abd::export_system(s, off, ij, cap));
+  if (off) CK(abd::export_system(s, off, ij, cap));
   CK(cudaStreamSynchronize(s.stream));
-  if (n_pairs) *n_pairs = s.n_pairs;
+  if (n_pairs) *n_pairs = s.sys_list ? s.x_n : s.n_pairs;
   return ABD_OK;
 }
 
@@ -1400,8 +1424,10 @@ int step_outcome(abd_sim* h) {
   s.n_adj = s.hstat[abd::DS_NADJ];
   const int bits = s.hstat[abd::DS_STATUS];
   if (!(bits & abd::kRerunMask)) {
-    s.sys_list = true;  // (abd_export_system makes the exact pairs when it is asked)
-    s.n_pairs = -1;
+    s.sys_list = true;  // (gather_system makes the exact pairs when a call asks for them)
+    s.sys_dhat = s.prm.dhat;
+    s.sys_friction = s.prm.friction_mu > 0.0 ? 1 : 0;
+    s.x_n = -1;
     return 0;
   }
   CK(cudaMemcpyAsync(s.dq, s.dq_save, sizeof(double) * 12 * s.n, cudaMemcpyDeviceToDevice, s.stream));
@@ -1543,6 +1569,7 @@ int step_device(abd_sim* h, const abd_states* stp, double* x_view, abd_step_info
   Sim& s = h->s;
   const abd_states& st = *stp;
   int r = ABD_OK;
+  s.sys_list = false;  // (until it is done: step_outcome)
   // a rerun restarts the whole step and meets the next short list, so a step gets the reruns of
   // all its passes; each recaptures (the buffers and capacities are in the key)
   for (int tries = 0;; ++tries) {
@@ -1701,6 +1728,7 @@ int abd_batch_step(abd_batch* b, const abd_states* st, double* const* x_view, ab
     }
     b->key = k.h;
   }
+  for (abd_sim* h : b->sims) h->s.sys_list = false;  // (until its step is done: step_outcome)
   CK(cudaGraphLaunch(b->exec, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   int first_error = ABD_OK;
