@@ -17,10 +17,9 @@
 
 #include <stdint.h>
 
-namespace abd {
+#include "abd_digits.cuh"
 
-constexpr int kXD = 10;      // 32-bit digits
-constexpr int kXB0 = -192;   // weight exponent of digit 0
+namespace abd {
 
 enum : long long { XS_NAN = 1, XS_PINF = 2, XS_NINF = 4, XS_RANGE = 8 };
 

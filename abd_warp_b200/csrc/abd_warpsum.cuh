@@ -13,12 +13,6 @@
 
 namespace abd {
 
-constexpr int kDW = 14;                                // bits of a digit
-constexpr int kDN = (32 * kXD + kDW - 1) / kDW;        // digits: 23
-constexpr int kDFlags = 31;                            // counter of the flags (XS_*)
-constexpr int kDSlots = 32;                            // counters of a sum
-constexpr int kDTerms = 1 << 17;                       // terms a set of counters holds
-
 // x into the counters s [kDSlots] (shared memory)
 __device__ inline void ds_add(int* s, double x) {
   const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
@@ -52,12 +46,12 @@ __device__ inline void ds_add(int* s, double x) {
 }
 
 // The carries of a set of counters to the counters above (one warp), which makes room for more
-// terms: after it, a counter is below 2^17 + 2^kDW in magnitude
+// terms: after it, a counter is at most 2^17 + 2^kDW in magnitude, with the sign of what it held
 __device__ inline void ds_fold(int* s) {
-  const int lane = (int)(threadIdx.x & 31), v = s[lane];
-  const int up = __shfl_up_sync(0xffffffffu, v >> kDW, 1);
+  const int lane = (int)(threadIdx.x & 31), v = s[lane], c = ds_carry(v);
+  const int up = __shfl_up_sync(0xffffffffu, c, 1);
   __syncwarp();
-  if (lane < kDFlags) s[lane] = (v & ((1 << kDW) - 1)) + (lane ? up : 0);
+  if (lane < kDFlags) s[lane] = v - c * (1 << kDW) + (lane ? up : 0);
 }
 
 // Counter i of the set s into the limbs (or flags) of an XSum in global memory (a thread per counter)
@@ -68,25 +62,26 @@ __device__ inline void ds_to_limbs(const int* s, int i, XSum* x) {
     atomicOr((unsigned long long*)&x->flags, (unsigned long long)v);
     return;
   }
-  const int j = kDW * i / 32, o = kDW * i % 32;
-  const long long w = (long long)v * (1LL << o);  // below 2^63
-  const bool top = j + 1 == kXD;                  // (the top limb takes all of it)
-  atomicAdd((unsigned long long*)&x->d[j], (unsigned long long)(top ? w : w & 0xffffffffLL));
-  if (!top) atomicAdd((unsigned long long*)&x->d[j + 1], (unsigned long long)(w >> 32));
+  if (i >= kDTop) {  // (no sum reaches it)
+    atomicOr((unsigned long long*)&x->flags, (unsigned long long)XS_RANGE);
+    return;
+  }
+  int j;
+  long long lo, hi;
+  ds_limb(i, v, j, lo, hi);
+  atomicAdd((unsigned long long*)&x->d[j], (unsigned long long)lo);
+  if (hi) atomicAdd((unsigned long long*)&x->d[j + 1], (unsigned long long)hi);
 }
 
 // The counters of the set s added to a register accumulator
 __device__ inline void ds_merge(XSum& x, const int* s) {
 #pragma unroll
-  for (int i = 0; i < kDN; ++i) {
-    const int j = kDW * i / 32, o = kDW * i % 32;
-    const long long w = (long long)s[i] * (1LL << o);  // below 2^63
-    if (j + 1 == kXD) {
-      x.d[j] += w;
-    } else {
-      x.d[j] += w & 0xffffffffLL;
-      x.d[j + 1] += w >> 32;
-    }
+  for (int i = 0; i < kDTop; ++i) {
+    int j;
+    long long lo, hi;
+    ds_limb(i, s[i], j, lo, hi);
+    x.d[j] += lo;
+    if (j + 1 < kXD) x.d[j + 1] += hi;
   }
   x.flags |= s[kDFlags];
 }
