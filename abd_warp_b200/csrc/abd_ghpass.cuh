@@ -8,11 +8,12 @@
 
 namespace abd {
 
-// The counters of a GH pass, cleared before it (by threads t of stride s)
+// The counters of a GH pass, cleared before it (by threads t of stride s).  Not the coupled pairs
+// (DS_NACTP): a solve after the step forms its clusters from the last pass's.
 __device__ inline void clear_gh(int* ds, int* pair_cand, int cap_pairs, int t, int s) {
   const int np = min(ds[DS_NPAIRS], cap_pairs);
   for (int p = t; p < np; p += s) pair_cand[4 * p + 1] = 0;
-  if (t == 0) ds[DS_PT_COUNT] = ds[DS_EE_COUNT] = ds[DS_VG_COUNT] = ds[DS_ACTIVE] = ds[DS_NCONTACT] = ds[DS_NACTP] = 0;
+  if (t == 0) ds[DS_PT_COUNT] = ds[DS_EE_COUNT] = ds[DS_VG_COUNT] = ds[DS_ACTIVE] = ds[DS_NCONTACT] = 0;
 }
 
 // contacts into their pair's segment, thread k taking contacts k, k + stride, ... (the order
@@ -201,7 +202,7 @@ __device__ inline bool gh_lag(const NarrowArgs& a) { return a.fric_lag && (!a.en
 // or vertex positions of its own: a thread computes its four positions and applies the culling
 // predicate (culling2.py:32-79, 213-227) as k_ls_eval does (linesearch.cu: the primitives' boxes;
 // the body boxes only where a tie at the rounding boundary leaves them to decide).  CTA 0 also
-// clears what the iteration's CCD pass and line search add to.
+// clears what the iteration's assembly, CCD pass and line search add to.
 // Bound by its chain of dependent loads (candidate, vertices, bodies, DOFs): 8.7 us for the 71k
 // candidates of the 1024-body pile, in place of 43 us (broad phase, pairs, and the scan of the
 // candidates kept from the CCD pass).
@@ -213,6 +214,7 @@ __device__ __forceinline__ void list_gh_pass(const NarrowArgs& a, int bx, int nb
     for (int i = threadIdx.x; i < kLsMax * (kXD + 1); i += T) reinterpret_cast<long long*>(a.ls_energy)[i] = 0;
     if (threadIdx.x == 0) {
       a.dstat[DS_NECAND] = 0;
+      a.dstat[DS_NACTP] = 0;  // (the assembly appends them)
       *a.toi_key = 0;
     }
   }

@@ -48,6 +48,7 @@ def _step(sim, o, prm):
     A, p = np.array(s["A0"]), np.array(s["p0"])
     ref = o.gh(A, p)
     dq0 = np.full((sim.n_bodies, 12), 1e-3)
+    solved = (dq0, *o.solve(dq0))
     # (a culling clears the list of coupled pairs: a solve after it has clusters of one body)
     o.set_params(dataclasses.replace(prm, precond=0))
     alone = (dq0, *o.solve(dq0))
@@ -55,7 +56,7 @@ def _step(sim, o, prm):
     o.set_state(*[s[k] for k in KEYS], dq=s["dq"])  # (solve leaves its solution as the warm start)
     sim.step()
     o.step()
-    return torch.as_tensor(A, device="cuda"), torch.as_tensor(p, device="cuda"), ref, alone
+    return torch.as_tensor(A, device="cuda"), torch.as_tensor(p, device="cuda"), ref, solved, alone
 
 
 def _same_system(sim, ref, solved):
@@ -81,14 +82,45 @@ def test_culling_at_the_same_dofs(before):
     sim, o, prm = _pair()
     blocks = 0
     for _ in range(3):
-        A, p, ref, alone = _step(sim, o, prm)
+        A, p, ref, solved, alone = _step(sim, o, prm)
         if before:
-            _export(sim)
+            _same_system(sim, ref, solved)
         sim.collision_set_dofs(A, p)
         _same_system(sim, ref, alone)
         _same_state(sim, o)
         blocks += int((np.abs(np.asarray(ref["off"])) > 0).any())
     assert blocks > 0
+
+
+@pytest.mark.parametrize("scenes_together", [1, 10])
+def test_solve_after_a_step(scenes_together):
+    """A solve of the step's last system has the pass's preconditioner clusters: alone and in a batch whose
+    scenes share a kernel."""
+    import torch
+    from abd_warp_b200.batch import BatchSimulator
+    sim, o, prm = _pair()
+    sims = [sim]
+    if scenes_together > 1:
+        batch = BatchSimulator([scenes.small_pile(2, 2, seed=21, level=1, radius=0.2)[0] for _ in range(scenes_together)], prm)
+        sims = batch.sims
+        for s in sims:
+            for k in KEYS:
+                getattr(s.states, k).copy_(getattr(sim.states, k))
+            s.dq = sim.dq
+    for _ in range(2):
+        s = o.get_state()
+        o.gh(s["A0"], s["p0"])
+        dq0 = np.full((sim.n_bodies, 12), 1e-3)
+        want, it = o.solve(dq0)
+        o.set_state(*[s[k] for k in KEYS], dq=s["dq"])
+        o.step()
+        if scenes_together > 1:
+            batch.step()
+        else:
+            sim.step()
+        for s in sims:
+            got, n = s.solve(torch.as_tensor(dq0, device="cuda"))
+            assert n == it and np.array_equal(got.cpu().numpy(), np.asarray(want).reshape(-1, 12))
 
 
 @pytest.mark.parametrize("call", ["static", "swept", "positions"])
