@@ -478,8 +478,9 @@ constexpr int kExt = 14;          // extreme vertices per body
 constexpr int kSlice = 96;        // vertices per warp of k_vertex_broad (three per lane)
 constexpr int kParK = 4;          // dpar slot of a batch's trial count
 constexpr int kParAlpha = 5;      // dpar slots of its step lengths
-constexpr int kParSkin = kParAlpha + kLsMax;  // dpar slot of the kept list's displacement
-constexpr int kNPar = kParSkin + 1;
+constexpr int kParSkin = kParAlpha + kLsMax;  // dpar slot of the kept list's displacement: what it was made with
+constexpr int kParSkinNext = kParSkin + 1;    // and of the next list's
+constexpr int kNPar = kParSkinNext + 1;
 
 // dstat layout
 enum : int {

@@ -46,8 +46,8 @@ struct NarrowArgs {
   const int* vbody;
   int cap_ecand;
   int4* ecand;                  // CCD_LS: line-search candidates
-  // CCD_LS making the kept list (list_build): its candidates with their pairs; the region's
-  // displacement dilates every box
+  // CCD_LS making the kept list (list_build): its candidates with their pairs; the displacement
+  // it is made with dilates every box
   int make_list;
   int cap_list;
   int4* list;

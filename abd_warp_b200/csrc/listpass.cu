@@ -16,7 +16,8 @@
 // in one to four steps (ten iterations each), in 55 to 110 us; 64 piled-up spheres, whose Newton
 // steps are long, make it every fourth iteration.
 //
-// The skin follows the scene: it doubles when an iteration leaves the region that the same step
+// The skin follows the scene (from list to list: the DOFs are checked against the one that the list in
+// use was made with): it doubles when an iteration leaves the region that the same step
 // made, while the list is short (a pass over 65k candidates takes about as long as one over 10k: a
 // thread each on 296 CTAs), and halves when the list is long (several candidates a thread).
 #include <cuda_runtime.h>
@@ -78,8 +79,8 @@ __global__ void k_region(int n, abd_params P, abd_states st, const double* dq, c
                                       __double2float_ru(0.5 * P.dhat) + __double2float_ru(*skin)));
 }
 
-// The list is made (unless a capacity was short: the step is run again): it may be used, and the
-// skin of the next one follows from this one.  Also the traversal's time (kernel profiling).
+// The list is made (unless a capacity was short: the step is run again): it may be used while the DOFs
+// stay within its own skin, and the skin of the next one follows from it.  Also the traversal's time (kernel profiling).
 __global__ void k_list_made(Mailbox* box, int* bad, double* dpar, double dhat, int cap_list, int prof_bytes) {
   StepDev& S = box->step;
   if (S.t1 > S.t0 && S.t0 != ~0ULL) {
@@ -98,9 +99,10 @@ __global__ void k_list_made(Mailbox* box, int* bad, double* dpar, double dhat, i
   *bad = 0;
   ++S.lists;
   const int m = min(box->dstat[DS_NLIST], cap_list);
-  const double skin = dpar[kParSkin];
-  if (S.resume && m <= kListShort) dpar[kParSkin] = fmin(2.0 * skin, kSkinMax * dhat);
-  else if (m > kListLong) dpar[kParSkin] = fmax(0.5 * skin, kSkinMin * dhat);
+  const double skin = dpar[kParSkinNext];
+  dpar[kParSkin] = skin;
+  if (S.resume && m <= kListShort) dpar[kParSkinNext] = fmin(2.0 * skin, kSkinMax * dhat);
+  else if (m > kListLong) dpar[kParSkinNext] = fmax(0.5 * skin, kSkinMin * dhat);
 }
 
 // Blocks [0, G): the list's candidates, one thread each; blocks [G, G + Gb): one thread per body;
@@ -123,8 +125,9 @@ __global__ void __launch_bounds__(128) k_list_ccd(const __grid_constant__ CcdArg
 
 cudaError_t list_build(Sim& s, const abd_states& st) {
   const bool fr = s.prm.friction_mu > 0.0;
-  k_region<<<blocks(s.n, 128), 128, 0, s.stream>>>(s.n, s.prm, st, s.dq, s.fixed, s.body_rest, s.dpar + kParSkin, s.reg,
-                                                  s.fdof, s.body_sup, s.chunk_act + s.nch, s.box, fr ? 1 : 0);
+  k_region<<<blocks(s.n, 128), 128, 0, s.stream>>>(s.n, s.prm, st, s.dq, s.fixed, s.body_rest,
+                                                  s.dpar + kParSkinNext, s.reg, s.fdof, s.body_sup, s.chunk_act + s.nch, s.box,
+                                                  fr ? 1 : 0);
   ++s.launches;
   cudaError_t e = list_pairs(s, fr ? s.fric_mask : nullptr);
   if (e == cudaSuccess) e = list_traverse(s);

@@ -76,7 +76,7 @@ NarrowArgs narrow_args(Sim& s, int mode, const double* A, const double* p, const
   a.make_list = 0;
   a.cap_list = s.cap_list;
   a.list = s.list;
-  a.skin = s.dpar + kParSkin;
+  a.skin = s.dpar + kParSkinNext;
   a.cap_ecand = s.cap_ecand;
   a.ecand = s.ecand;
   a.cap_contacts = s.cap_contacts;

@@ -887,7 +887,7 @@ int abd_sim_create(const abd_scene_desc* d, const abd_params* prm, void* stream,
   if (e == cudaSuccess) {  // dpar = {trial step, 1 (the full step of the CCD bound), 0, ...}
     for (int k = 0; k < abd::kNPar; ++k) s.hpar[k] = 0.0;
     s.hpar[1] = 1.0;
-    s.hpar[abd::kParSkin] = kSkin0 * prm->dhat;
+    s.hpar[abd::kParSkinNext] = kSkin0 * prm->dhat;
     e = cudaMemcpyAsync(s.dpar, s.hpar, abd::kNPar * sizeof(double), cudaMemcpyHostToDevice, s.stream);
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(s.red_count, 0, sizeof(int) * abd::kRedSlots, s.stream);
@@ -964,9 +964,9 @@ int abd_sim_set_params(abd_sim* h, const abd_params* prm) {
   if (int r = drop_superset(h)) return r;
   // the kept list belongs to the old parameters; its skin starts again
   CK(cudaMemsetAsync(h->s.dint + abd::kListBad, 1, sizeof(int), h->s.stream));
-  h->s.hpar[abd::kParSkin] = kSkin0 * prm->dhat;
-  CK(cudaMemcpyAsync(h->s.dpar + abd::kParSkin, h->s.hpar + abd::kParSkin, sizeof(double), cudaMemcpyHostToDevice,
-                     h->s.stream));
+  h->s.hpar[abd::kParSkinNext] = kSkin0 * prm->dhat;
+  CK(cudaMemcpyAsync(h->s.dpar + abd::kParSkinNext, h->s.hpar + abd::kParSkinNext, sizeof(double),
+                     cudaMemcpyHostToDevice, h->s.stream));
   h->s.prm = *prm;
   ++h->s.prm_version;  // parameters are kernel arguments of the captured passes
   return ABD_OK;
