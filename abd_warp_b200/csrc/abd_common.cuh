@@ -235,11 +235,17 @@ struct FricRec {
   int I, J, kind, pad;
 };
 
+// kernels of a captured step's loop bodies: of a Newton iteration, of making the list
+struct LoopLaunches {
+  long long step = 0, list = 0;
+};
+
 // one captured pass (see abd_graph.cuh)
 struct GraphSlot {
   cudaGraphExec_t exec = nullptr;
   uint64_t key = 0;
   long long nlaunch = 0;  // kernels per replay
+  LoopLaunches loop;      // (a step: also of its loops' bodies, which nlaunch counts once)
 };
 
 struct Sim {
@@ -351,7 +357,7 @@ struct Sim {
   cudaStream_t cap_stream5 = nullptr;  // captures that IF node's body
   bool in_device_loop = false;
   double* dq_save = nullptr;       // [12 n] dq at the start of a device-loop step (for a rerun)
-  long long step_launch = 0, list_launch = 0;  // kernels of a Newton iteration, of making the list
+  LoopLaunches loop;               // of the step that is being captured
   int gh_energy = 0;               // the GH pass also sums the energy at its DOFs
   int exact_hessian = 0;           // the GH pass assembles the exact Hessian (the adjoint's)
   const int* energy_gate = nullptr;  // device loop: the GH pass sums the energy only while this

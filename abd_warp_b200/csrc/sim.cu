@@ -38,6 +38,7 @@ struct abd_batch {
   cudaGraphExec_t exec = nullptr;
   uint64_t key = 0;
   std::vector<long long> top;         // kernels of each branch outside its loops
+  std::vector<abd::LoopLaunches> loop;  // and of its loops
   // the small scenes whose Newton iterations share a kernel (newton_batch.cu)
   std::vector<int> joint;
   void* args = nullptr;               // their arguments (device)
@@ -1374,7 +1375,7 @@ int step_issue(abd_sim* h, const abd_states& st, double* x_view) {
           return ABD_OK;
         }))
       return q;
-    s.list_launch = s.launches - l0;
+    s.loop.list = s.launches - l0;
     if (int q = abd::add_conditional(s.stream, hn, cudaGraphCondTypeWhile, &nbody)) return q;
     const long long l1 = s.launches;
     if (int q = abd::capture_body(s, nbody, s.cap_stream4, [&]() -> int {
@@ -1383,7 +1384,7 @@ int step_issue(abd_sim* h, const abd_states& st, double* x_view) {
           return ABD_OK;
         }))
       return q;
-    s.step_launch = s.launches - l1;
+    s.loop.step = s.launches - l1;
     CK(abd::round_end(s, hr));
     return ABD_OK;
   });
@@ -1415,11 +1416,12 @@ constexpr int kHostFinish = -2;
 // 0 when the step is complete; kRerun when a list overflowed (the warm start restored, the
 // kept candidates dropped, the list grown: run the step again); kHostFinish when a line search
 // needed more trials (likewise restored: the host loop finishes the step); or an ABD error.
-int step_outcome(abd_sim* h) {
+// loop: the kernels of that graph's loops
+int step_outcome(abd_sim* h, const abd::LoopLaunches& loop) {
   Sim& s = h->s;
   std::memcpy(s.hstat, s.hbox->dstat, sizeof(int) * abd::DS_NSLOTS);
   const abd::StepDev& S = s.hbox->step;
-  s.launches += (long long)S.it * s.step_launch + (long long)S.lists * s.list_launch;
+  s.launches += (long long)S.it * loop.step + (long long)S.lists * loop.list;
   s.n_pairs = s.hstat[abd::DS_NPAIRS];
   s.n_adj = s.hstat[abd::DS_NADJ];
   const int bits = s.hstat[abd::DS_STATUS];
@@ -1535,8 +1537,9 @@ int joint_issue(abd_batch* b, const abd_states* st, double* const* x_view, std::
                 return ABD_OK;
               }))
             return q;
-          s.list_launch = s.launches - l0;
-          s.step_launch = 0;  // (an iteration has no kernels of its own)
+          s.loop.list = s.launches - l0;
+          s.loop.step = 0;  // (an iteration has no kernels of its own)
+          b->loop[b->joint[k]] = s.loop;
           s.launches = l0;
           CK(cudaEventRecord(s.fork_ev[1], s.stream));
           CK(cudaStreamWaitEvent(b->body, s.fork_ev[1], 0));
@@ -1575,12 +1578,16 @@ int step_device(abd_sim* h, const abd_states* stp, double* x_view, abd_step_info
   for (int tries = 0;; ++tries) {
     step_modes(s, true);
     const long long launches0 = s.launches;
-    r = abd::run_graph(s, s.g_step, step_key(s, st, x_view), [&]() { return step_issue(h, st, x_view); });
+    r = abd::run_graph(s, s.g_step, step_key(s, st, x_view), [&]() {
+      const int q = step_issue(h, st, x_view);
+      s.g_step.loop = s.loop;
+      return q;
+    });
     step_modes(s, false);
     if (r) return r;
-    s.launches = launches0 + s.g_step.nlaunch - s.step_launch - s.list_launch;  // the loops: step_outcome
+    s.launches = launches0 + s.g_step.nlaunch - s.g_step.loop.step - s.g_step.loop.list;  // (step_outcome)
     CK(cudaStreamSynchronize(s.stream));
-    r = step_outcome(h);
+    r = step_outcome(h, s.g_step.loop);
     if (r == 0) break;
     if (r == kHostFinish) return step_host(h, stp, x_view, info);
     if (r > 0) return r;
@@ -1633,6 +1640,7 @@ int abd_batch_create(int n, abd_sim* const* sims, void* stream, abd_batch** out)
   b->branch.assign(n, nullptr);
   b->join.assign(n, nullptr);
   b->top.assign(n, 0);
+  b->loop.assign(n, {});
   cudaError_t e = ABD_NOTE(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking));
   if (e == cudaSuccess) e = ABD_NOTE(cudaStreamCreateWithFlags(&b->body, cudaStreamNonBlocking));
   if (e == cudaSuccess) e = ABD_NOTE(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
@@ -1704,7 +1712,8 @@ int abd_batch_step(abd_batch* b, const abd_states* st, double* const* x_view, ab
       r = step_issue(b->sims[i], st[i], x_view ? x_view[i] : nullptr);
       step_modes(s, false);
       s.stream = saved;
-      b->top[i] = s.launches - l0 - s.step_launch - s.list_launch;
+      b->top[i] = s.launches - l0 - s.loop.step - s.loop.list;
+      b->loop[i] = s.loop;
       s.launches = l0;
       if (r == ABD_OK && (ABD_NOTE(cudaEventRecord(b->join[i], b->branch[i])) != cudaSuccess ||
                           ABD_NOTE(cudaStreamWaitEvent(b->cap, b->join[i], 0)) != cudaSuccess))
@@ -1735,7 +1744,7 @@ int abd_batch_step(abd_batch* b, const abd_states* st, double* const* x_view, ab
   for (int i = 0; i < n; ++i) {
     abd_sim* h = b->sims[i];
     h->s.launches += b->top[i];
-    int r = step_outcome(h);
+    int r = step_outcome(h, b->loop[i]);
     abd_step_info* inf = info ? info + i : nullptr;
     if (r == 0) r = step_info(h, inf);
     else if (r == kRerun) r = step_device(h, &st[i], x_view ? x_view[i] : nullptr, inf);  // alone, grown
