@@ -326,6 +326,7 @@ struct Sim {
   int cap_list = 0;
   int4* list = nullptr;            // (type, primitive a, primitive b, pair)
   double* reg = nullptr;
+  double body_size = 0.0;          // the free bodies' mean half extent (host)
   int* ext = nullptr;              // [n][kExt] vertices extreme in fixed rest-frame directions
   double* gh_q = nullptr;          // [12 n] the DOFs (A, then p) of the device loop's last GH pass
   // the device loop's last GH pass numbered its body pairs by the list (and nothing has replaced that
@@ -430,6 +431,12 @@ struct Sim {
   unsigned long long* dmin = nullptr;  // = &box->toi_key
 };
 
+// the unit of the kept list's displacement (listpass.cu says why)
+inline double skin_unit(const Sim& s, double dhat) {
+  const double h = s.body_size / 64.0, least = dhat / 16.0;
+  return h < least ? least : h < dhat ? h : dhat;
+}
+
 // CTAs of a grid-stride pass over a scene's candidates, whose number only the device knows: one per
 // `per` primitives of the scene, from 8 to `most`.  (Launching CTAs costs: many scenes stepped
 // together spent most of their time on CTAs without work.)
@@ -520,6 +527,7 @@ struct StepDev {
   int run;           // (batches) the scene takes part in the round
   int lists;         // candidate lists made
   int rounds;        // rounds begun
+  int shrunk;        // a list over its capacity was made smaller, not its capacity larger
   double E0, E1;     // energy of the current iterate and of the accepted one
   double alpha, toi; // the last accepted step length and raw time of impact
   unsigned long long t0, t1;       // first start and last end (ns) of the current narrow launch

@@ -19,8 +19,15 @@
 // The skin follows the scene (from list to list: the DOFs are checked against the one that the list in
 // use was made with): it doubles when an iteration leaves the region that the same step
 // made, while the list is short (a pass over 65k candidates takes about as long as one over 10k: a
-// thread each on 296 CTAs), and halves when the list is long (several candidates a thread).
+// thread each on 296 CTAs), and halves when the list is long (several candidates a thread; the next step
+// then makes the list again).  A list that is very long for its scene is not given the memory: the step
+// starts again with half the skin, down to the least one.  The skin is counted in units of dhat, or of
+// 1/64 of the bodies' half extent where that is less: with dhat in place of it, 28 bodies of 0.2 m with
+// dhat = 60 mm made lists of 20 GB and took 340 ms a step (2.2 ms without a list).
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <climits>
 
 #include "abd_listccd.cuh"
 
@@ -33,7 +40,7 @@ namespace {
 inline unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 constexpr int kListShort = 1 << 16, kListLong = 1 << 18;  // candidates: the skin may grow below, shrinks above
-constexpr double kSkinMin = 1.0, kSkinMax = 64.0;         // in units of dhat
+constexpr double kSkinMin = 1.0, kSkinMax = 64.0;         // in skin units (Sim::skin_unit)
 
 // The list's region around the step: its segment runs from the iterate q to q - dq when an
 // iteration asked for the list (its solve is done), else, at the step's start, to the prediction
@@ -81,8 +88,11 @@ __global__ void k_region(int n, abd_params P, abd_states st, const double* dq, c
 
 // The list is made (unless a capacity was short: the step is run again): it may be used while the DOFs
 // stay within its own skin, and the skin of the next one follows from it.  Also the traversal's time (kernel profiling).
-__global__ void k_list_made(Mailbox* box, int* bad, double* dpar, double dhat, int cap_list, int prof_bytes) {
+// unit: of the skin; very_long: candidates
+__global__ void k_list_made(Mailbox* box, int* bad, double* dpar, double unit, int cap_list, int very_long,
+                            int prof_bytes) {
   StepDev& S = box->step;
+  const double skin = dpar[kParSkinNext];
   if (S.t1 > S.t0 && S.t0 != ~0ULL) {
     S.prof_ns += S.t1 - S.t0;
     ++S.prof_n;
@@ -95,14 +105,20 @@ __global__ void k_list_made(Mailbox* box, int* bad, double* dpar, double dhat, i
   }
   S.t0 = ~0ULL;
   S.t1 = 0ULL;
-  if (box->dstat[DS_STATUS] & kRerunMask) return;
+  if (box->dstat[DS_STATUS] & kRerunMask) {
+    if ((box->dstat[DS_STATUS] & ST_LIST_OVERFLOW) && (unsigned)box->dstat[DS_NLIST] > (unsigned)very_long &&
+        skin > kSkinMin * unit) {
+      dpar[kParSkinNext] = fmax(0.5 * skin, kSkinMin * unit);
+      S.shrunk = 1;  // (the host does not grow the list)
+    }
+    return;
+  }
   *bad = 0;
   ++S.lists;
   const int m = min(box->dstat[DS_NLIST], cap_list);
-  const double skin = dpar[kParSkinNext];
   dpar[kParSkin] = skin;
-  if (S.resume && m <= kListShort) dpar[kParSkinNext] = fmin(2.0 * skin, kSkinMax * dhat);
-  else if (m > kListLong) dpar[kParSkinNext] = fmax(0.5 * skin, kSkinMin * dhat);
+  if (S.resume && m <= kListShort) dpar[kParSkinNext] = fmin(2.0 * skin, kSkinMax * unit);
+  else if (m > kListLong) dpar[kParSkinNext] = fmax(0.5 * skin, kSkinMin * unit);
 }
 
 // Blocks [0, G): the list's candidates, one thread each; blocks [G, G + Gb): one thread per body;
@@ -132,7 +148,10 @@ cudaError_t list_build(Sim& s, const abd_states& st) {
   cudaError_t e = list_pairs(s, fr ? s.fric_mask : nullptr);
   if (e == cudaSuccess) e = list_traverse(s);
   if (e != cudaSuccess) return e;
-  k_list_made<<<1, 1, 0, s.stream>>>(s.box, s.dint + kListBad, s.dpar, s.prm.dhat, s.cap_list, s.prof_on == 2 ? 1 : 0);
+  // (32 MB for a small scene's list and its line-search candidates)
+  const int very_long = (int)std::min((long long)INT_MAX, std::max(1LL << 20, 2 * ((long long)s.V + s.E)));
+  k_list_made<<<1, 1, 0, s.stream>>>(s.box, s.dint + kListBad, s.dpar, skin_unit(s, s.prm.dhat), s.cap_list, very_long,
+                                     s.prof_on == 2 ? 1 : 0);
   ++s.launches;
   return cudaGetLastError();
 }

@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(CT, 5) k_chunk_narrow(NarrowArgs a) {
       cbuf[k] = rec;
     } else {
       const int pos = append_slot(ccount);
-      if (pos < ccap) cdst[pos] = rec;
+      if ((unsigned)pos < (unsigned)ccap) cdst[pos] = rec;
       else atomicOr(&a.dstat[DS_STATUS], cflag);
     }
   };
@@ -640,7 +640,7 @@ __global__ void __launch_bounds__(CT, 5) k_chunk_narrow(NarrowArgs a) {
     if (tid == 0) cbase = atomicAdd(ccount, n);
     __syncthreads();
     for (int e = tid; e < n; e += CT) {
-      if (cbase + e < ccap) cdst[cbase + e] = cbuf[e];
+      if ((unsigned)(cbase + e) < (unsigned)ccap) cdst[cbase + e] = cbuf[e];
       else atomicOr(&a.dstat[DS_STATUS], cflag);
     }
     __syncthreads();

@@ -36,8 +36,9 @@ namespace {
 // in the kept list's region; thread 0 clears the step's counters and enters the round loop.
 __global__ void k_step_begin(Mailbox* box, cudaGraphConditionalHandle h, int n, abd_states st, const double* dq,
                              double* dq_save, abd_params P, const int* fixed, const double* reg, const Box* body_rest,
-                             const double* skin, int* bad) {
+                             const double* dpar, int* bad) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  const double skin = dpar[kParSkin];
   if (b < n) {
     for (int k = 0; k < 9; ++k) st.A[9 * b + k] = st.Ak[9 * b + k] = st.A0[9 * b + k];
     for (int k = 0; k < 3; ++k) st.p[3 * b + k] = st.pk[3 * b + k] = st.p0[3 * b + k];
@@ -46,19 +47,20 @@ __global__ void k_step_begin(Mailbox* box, cudaGraphConditionalHandle h, int n, 
     load_dofs(st.A0, st.p0, b, M);
     const Box R = load_box(&body_rest[b]);
     const double* g = reg + 24 * (size_t)b;
-    bool in = in_region(g, M, R, *skin);
+    bool in = in_region(g, M, R, skin);
     if (in && !fixed[b]) {
       tilde_of(P, st, b, M, M + 9);
-      in = in_region(g, M, R, *skin);
+      in = in_region(g, M, R, skin);
     }
     if (!in) *bad = 1;
   }
   if (b != 0) return;
+  if (dpar[kParSkinNext] < skin) *bad = 1;  // (the list was long)
   xs_zero(box->energy);
   StepDev& S = box->step;
   S.it = S.lin = S.ls = 0;
   S.n_pt = S.n_ee = S.n_vg = S.n_ij = S.n_active = 0;
-  S.resume = S.again = S.lists = S.rounds = 0;
+  S.resume = S.again = S.lists = S.rounds = S.shrunk = 0;
   S.run = 1;
   S.E0 = S.E1 = S.alpha = 0.0;
   S.toi = 1.0;
@@ -203,7 +205,7 @@ cudaError_t adjoint_out(Sim& s, const double* lam, const double* qdb, double* qb
 
 cudaError_t step_begin(Sim& s, const abd_states& st, cudaGraphConditionalHandle h) {
   k_step_begin<<<(s.n + 127) / 128, 128, 0, s.stream>>>(s.box, h, s.n, st, s.dq, s.dq_save, s.prm, s.fixed, s.reg,
-                                                        s.body_rest, s.dpar + kParSkin, s.dint + kListBad);
+                                                        s.body_rest, s.dpar, s.dint + kListBad);
   ++s.launches;
   return cudaGetLastError();
 }

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -197,14 +198,17 @@ int grow_ecand(Sim& s, int need) {
   return ABD_OK;
 }
 
-// the kept list, and room for all of it among the line-search candidates
+// the kept list, and room for all of it among the line-search candidates (need < 0: past 2^31)
 int grow_list(Sim& s, int need) {
   ++s.cap_gen;  // every captured pass is keyed on it
+  if (need < 0) return ABD_ERR_OVERFLOW;
   if (need > s.cap_list) {
+    const int cap = (int)std::min((long long)INT_MAX, std::max(need + need / 2LL, 2LL * s.cap_list));
     if (s.list) cudaFree(s.list);
     s.list = nullptr;
-    s.cap_list = std::max(need + need / 2, 2 * s.cap_list);
-    if (dalloc(&s.list, s.cap_list)) return ABD_ERR_OVERFLOW;
+    s.cap_list = 0;  // (no memory: no capacity)
+    if (dalloc(&s.list, cap)) return ABD_ERR_OVERFLOW;
+    s.cap_list = cap;
   }
   return grow_ecand(s, s.cap_list);
 }
@@ -286,7 +290,7 @@ int sync_read(Sim& s) {
 
 constexpr int kRerun = -1;
 
-constexpr double kSkin0 = 8.0;  // first skin of the kept candidate list, in units of dhat (listpass.cu adapts it)
+constexpr double kSkin0 = 8.0;  // first skin of the kept candidate list, in its units (listpass.cu adapts it)
 
 // After sync_read: grow every capacity whose overflow bit is set and clear those bits.
 // Returns kRerun when the pass has to be rerun, 0 when it is complete, or an ABD error.
@@ -312,7 +316,7 @@ int overflow(Sim& s) {
   if (!r && (bits & abd::ST_CCD_OVERFLOW)) r = grow_ccd(s, s.hstat[abd::DS_NCCD]);
   if (!r && (bits & abd::ST_ECAND_OVERFLOW)) r = grow_ecand(s, s.hstat[abd::DS_NECAND]);
   if (!r && (bits & abd::ST_FRIC_OVERFLOW)) r = grow_fric(s, s.hstat[abd::DS_NFRIC]);
-  if (!r && (bits & abd::ST_LIST_OVERFLOW)) r = grow_list(s, s.hstat[abd::DS_NLIST]);
+  if (!r && (bits & abd::ST_LIST_OVERFLOW) && !s.hbox->step.shrunk) r = grow_list(s, s.hstat[abd::DS_NLIST]);
   if (r) return r;
   const int clear = bits & ~mask;
   s.hstat[abd::DS_STATUS] = clear;
@@ -788,6 +792,15 @@ int abd_sim_create(const abd_scene_desc* d, const abd_params* prm, void* stream,
       }
     }
     ok(upload(&s.body_rest, brest.data(), brest.size(), s.stream));
+    int nfree = 0;
+    for (int b = 0; b < n; ++b) {
+      if (d->fixed[b]) continue;
+      double ext = 0.0;
+      for (int k = 0; k < 3; ++k) ext = std::max(ext, (double)brest[b].hi[k] - (double)brest[b].lo[k]);
+      s.body_size += 0.5 * ext;
+      ++nfree;
+    }
+    s.body_size = nfree ? s.body_size / nfree : INFINITY;
     // each body's vertices extreme in kExt fixed directions (the axes and the cube's diagonals)
     std::vector<int> ext((size_t)n * abd::kExt);
     const double dir[abd::kExt / 2][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 1, 1}, {1, 1, -1}, {1, -1, 1}, {-1, 1, 1}};
@@ -888,7 +901,7 @@ int abd_sim_create(const abd_scene_desc* d, const abd_params* prm, void* stream,
   if (e == cudaSuccess) {  // dpar = {trial step, 1 (the full step of the CCD bound), 0, ...}
     for (int k = 0; k < abd::kNPar; ++k) s.hpar[k] = 0.0;
     s.hpar[1] = 1.0;
-    s.hpar[abd::kParSkinNext] = kSkin0 * prm->dhat;
+    s.hpar[abd::kParSkinNext] = kSkin0 * abd::skin_unit(s, prm->dhat);
     e = cudaMemcpyAsync(s.dpar, s.hpar, abd::kNPar * sizeof(double), cudaMemcpyHostToDevice, s.stream);
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(s.red_count, 0, sizeof(int) * abd::kRedSlots, s.stream);
@@ -965,7 +978,7 @@ int abd_sim_set_params(abd_sim* h, const abd_params* prm) {
   if (int r = drop_superset(h)) return r;
   // the kept list belongs to the old parameters; its skin starts again
   CK(cudaMemsetAsync(h->s.dint + abd::kListBad, 1, sizeof(int), h->s.stream));
-  h->s.hpar[abd::kParSkinNext] = kSkin0 * prm->dhat;
+  h->s.hpar[abd::kParSkinNext] = kSkin0 * abd::skin_unit(h->s, prm->dhat);
   CK(cudaMemcpyAsync(h->s.dpar + abd::kParSkinNext, h->s.hpar + abd::kParSkinNext, sizeof(double),
                      cudaMemcpyHostToDevice, h->s.stream));
   h->s.prm = *prm;
