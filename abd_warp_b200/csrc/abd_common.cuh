@@ -235,9 +235,10 @@ struct FricRec {
   int I, J, kind, pad;
 };
 
-// kernels of a captured step's loop bodies: of a Newton iteration, of making the list
+// kernels of a captured step's loop bodies: of a Newton iteration, of making the list, of an iteration
+// of a large solve
 struct LoopLaunches {
-  long long step = 0, list = 0;
+  long long step = 0, list = 0, solve = 0;
 };
 
 // one captured pass (see abd_graph.cuh)
@@ -347,6 +348,7 @@ struct Sim {
   cudaStream_t cap_stream2 = nullptr;  // side branches
   GraphSlot g_ccd, g_ccd_ev, g_gh, g_gh0, g_ls, g_ls_dev;
   GraphSlot g_step;                // a whole time step as a device loop
+  GraphSlot g_solve, g_solve_dq;   // large solves (of adj_x, of dq)
   double* adj_x = nullptr;         // [12 n] the adjoint solve's unknown lambda
   cudaStream_t cap_stream3 = nullptr, cap_stream4 = nullptr;  // capture the loop's bodies
   // side branches of a pass (the GH pass's clustering, the host loop's dot products): a stream
@@ -404,12 +406,13 @@ struct Sim {
 
   // Newton system
   double *g = nullptr, *dq = nullptr, *diag = nullptr;  // [n][12], [n][12], [n][144]
-  // the Krylov solve (krylov.cu): published vectors [3][12 n], active neighbours [cap_adj], the
-  // rows' vectors [6][12 n] and positions [n] when they do not fit shared memory, and the most
-  // CTAs of its cluster
-  double *kry_pub = nullptr, *kry_spill = nullptr;
+  // the Krylov solve (krylov.cu): published vectors [3][12 n], active neighbours [cap_adj], and the
+  // most CTAs of its cluster; a large solve's (krylov_large.cu) vectors [8][12 n], scalars [32] and
+  // counters [4]
+  double* kry_pub = nullptr;
   int2* nb_act = nullptr;
-  void* kry_pos = nullptr;
+  double *kry_vec = nullptr, *kry_scal = nullptr;
+  int* kry_int = nullptr;
   int max_cluster = 1;
   int max_loop_ctas = 0;           // most CTAs of a scene's cluster in a batch's Newton loop (0: none)
   // preconditioner clusters (contact-coupled bodies, <= cluster_max each), formed on the
@@ -673,9 +676,12 @@ int krylov_outcome(Sim& s);
 // Enqueues a solve of the device-driven Newton loop: its outcome goes to the mailbox's step
 // counters, x.g and g.g to its dots
 int krylov_issue(Sim& s, double* x);
-cudaError_t prepare_krylov(Sim& s);               // kernel attributes (once, at creation)
+cudaError_t prepare_krylov(Sim& s);               // kernel attributes, a large solve's buffers (once, at creation)
 constexpr int kKrylovSmem = 196 * 1024;           // its most dynamic shared memory
-size_t krylov_pos_bytes(int n);
+bool krylov_is_large(const Sim& s);               // krylov_large.cu takes it:
+// the same solve by kernels over the whole GPU, for systems that one cluster is slow for
+int krylov_large_kernels(const Sim& s);           // of an iteration
+int krylov_large_issue(Sim& s, double* x, bool tally);
 
 // newton.cu: the kernels of the device-driven Newton loop (abd_step when the parameters'
 // newton_loop is 0).  Each enqueues on s.stream.

@@ -37,9 +37,6 @@ struct KrylovArgs {
   double tol2;
   double* x;                // in: the warm start, out: the solution
   double *pub0, *pub1, *pub2;  // published vectors (read by other rows): PCG p, p, z; BiCGSTAB y, z
-  double* spill;            // rows' vectors when they do not fit shared memory: [6][12 n]
-  PosInfo* spill_pos;       // [n]
-  int in_smem;
   int rows_max, pos_max;    // shared memory's rows and positions
   int* dstat;
   Mailbox* tally;           // device loop: the outcome goes to the step's counters, with
@@ -236,10 +233,10 @@ __device__ __forceinline__ void solve(const KrylovArgs& a, double* dyn, RedShare
   __syncthreads();
   const int P0 = sh_p[0], np = sh_p[1] - P0;
   c.nrow = 12 * np;
-  auto vec = [&](int k) { return a.in_smem ? dyn + (size_t)k * a.rows_max : a.spill + (size_t)k * 12 * n + 12 * (size_t)P0; };
+  auto vec = [&](int k) { return dyn + (size_t)k * a.rows_max; };
   double *const S_x = vec(0), *const S_r = vec(1), *const S_p = vec(2), *const S_a = vec(3);
   double *const S_v = PCG ? nullptr : vec(4), *const S_t = PCG ? nullptr : vec(5);
-  PosInfo* const pos = a.in_smem ? reinterpret_cast<PosInfo*>(dyn + (size_t)(PCG ? 4 : 6) * a.rows_max) : a.spill_pos + P0;
+  PosInfo* const pos = reinterpret_cast<PosInfo*>(dyn + (size_t)(PCG ? 4 : 6) * a.rows_max);
   // positions (a thread each)
   for (int q = c.tid; q < np; q += c.T) {
     const int b = a.cl_body[P0 + q], k = a.body_cl[b], base = a.cl_ptr[k];

@@ -26,6 +26,7 @@
 #include <map>
 #include <mutex>
 
+#include "abd_graph.cuh"
 #include "abd_krylov.cuh"
 
 namespace abd {
@@ -61,17 +62,12 @@ KrylovArgs krylov_args(Sim& s, double* x, bool tally, int C, size_t* smem_out) {
   a.pub0 = s.kry_pub;
   a.pub1 = s.kry_pub + 12 * (size_t)s.n;
   a.pub2 = s.kry_pub + 24 * (size_t)s.n;
-  a.spill = s.kry_spill;
-  a.spill_pos = reinterpret_cast<PosInfo*>(s.kry_pos);
   a.dstat = s.dstat;
   a.tally = tally ? s.box : nullptr;
   // a CTA's share, plus the members its last cluster may reach over it
   a.pos_max = std::min(s.n, (s.n + C - 1) / C + kMaxCluster);
   a.rows_max = 12 * a.pos_max;
-  size_t smem = (size_t)a.rows_max * (pcg ? 4 : 6) * sizeof(double) + (size_t)a.pos_max * sizeof(PosInfo);
-  a.in_smem = smem <= (size_t)kKrylovSmem ? 1 : 0;
-  if (!a.in_smem) smem = 0;
-  *smem_out = smem;
+  *smem_out = (size_t)a.rows_max * (pcg ? 4 : 6) * sizeof(double) + (size_t)a.pos_max * sizeof(PosInfo);
   return a;
 }
 
@@ -145,7 +141,19 @@ cudaError_t fit_cluster(K kernel, int* best) {
 
 }  // namespace
 
-size_t krylov_pos_bytes(int n) { return sizeof(PosInfo) * (size_t)n; }
+// Which solves are made by krylov_large.cu's kernels: more than kLargeBodies bodies (or, where the device
+// holds smaller clusters, vectors that do not fit them).  Below, this file's cluster is the faster one
+// for the few iterations that a step's solves take and for many: with 2,117 bodies a solve of two CG
+// iterations takes 128 us and each further one 20 us (377 and 29 us there, in round figures the cost of its
+// launches); with 4,097 bodies 178 and 193 us; 5,001 205 and 209; 8,101 300 (67 us an iteration) and 267 (50);
+// 16,385 566 (130) and 424 (73).  BiCGSTAB the same: 8,101 bodies 341 (157 us an iteration) and 282 (114).
+constexpr int kLargeBodies = 4096;
+bool krylov_is_large(const Sim& s) {
+  if (s.n > kLargeBodies) return true;
+  const int C = cluster_ctas(s);
+  const size_t pos = std::min(s.n, (s.n + C - 1) / C + kMaxCluster);
+  return pos * (12 * 6 * sizeof(double) + sizeof(PosInfo)) > (size_t)kKrylovSmem;  // (BiCGSTAB's)
+}
 
 cudaError_t prepare_krylov(Sim& s) {
   // the kernels' attributes and the largest cluster are the device's: found once per device (the
@@ -165,16 +173,28 @@ cudaError_t prepare_krylov(Sim& s) {
     best = c;
   }
   s.max_cluster = best;
-  return cudaSuccess;
+  if (!krylov_is_large(s)) return cudaSuccess;
+  e = cudaMalloc(&s.kry_vec, sizeof(double) * 96 * (size_t)s.n);
+  if (e == cudaSuccess) e = cudaMalloc(&s.kry_scal, sizeof(double) * 32);
+  if (e == cudaSuccess) e = cudaMalloc(&s.kry_int, sizeof(int) * 4);
+  return e;
 }
 
 int krylov_solve(Sim& s, double* x, int* iters_out) {
-  // (the kernel loads x in 16-byte pieces)
-  double* const y = reinterpret_cast<uintptr_t>(x) % 16 == 0 ? x : s.adj_x;
+  const bool large = krylov_is_large(s);
+  // (the kernel loads x in 16-byte pieces; a large solve's graph is kept for its own vectors)
+  double* const y = x == s.dq || (!large && reinterpret_cast<uintptr_t>(x) % 16 == 0) ? x : s.adj_x;
   const size_t bytes = sizeof(double) * 12 * (size_t)s.n;
   if (y != x && ABD_NOTE(cudaMemcpyAsync(y, x, bytes, cudaMemcpyDeviceToDevice, s.stream)) != cudaSuccess)
     return ABD_ERR_CUDA;
-  if (ABD_NOTE(enqueue(s, y, false)) != cudaSuccess) return ABD_ERR_CUDA;
+  if (large) {
+    KeyHash k;
+    k.add(y).add(s.prm_version).add(s.prm.solver).add(s.cap_gen);
+    if (int r = run_graph(s, y == s.dq ? s.g_solve_dq : s.g_solve, k.h, [&]() { return krylov_large_issue(s, y, false); }))
+      return r;
+  } else if (ABD_NOTE(enqueue(s, y, false)) != cudaSuccess) {
+    return ABD_ERR_CUDA;
+  }
   if (y != x && ABD_NOTE(cudaMemcpyAsync(x, y, bytes, cudaMemcpyDeviceToDevice, s.stream)) != cudaSuccess)
     return ABD_ERR_CUDA;
   if (!iters_out) return ABD_OK;
@@ -185,11 +205,17 @@ int krylov_solve(Sim& s, double* x, int* iters_out) {
   return ABD_OK;
 }
 
-int krylov_issue(Sim& s, double* x) { return ABD_NOTE(enqueue(s, x, true)) == cudaSuccess ? ABD_OK : ABD_ERR_CUDA; }
+int krylov_issue(Sim& s, double* x) {
+  if (!krylov_is_large(s)) return ABD_NOTE(enqueue(s, x, true)) == cudaSuccess ? ABD_OK : ABD_ERR_CUDA;
+  if (int r = krylov_large_issue(s, x, true)) return r;
+  s.loop.solve = krylov_large_kernels(s);
+  return ABD_NOTE(dots(s, x, s.g, s.g, s.g, s.box->dots, s.stream)) == cudaSuccess ? ABD_OK : ABD_ERR_CUDA;
+}
 
 int krylov_outcome(Sim& s) {
   const int* ds = s.hbox->dstat;
   if (!(ds[krylov::DS_R_DONE] || ds[krylov::DS_S_DONE])) s.host_status |= ST_SOLVER_NOCONV;
+  if (krylov_is_large(s)) s.launches += (long long)krylov_large_kernels(s) * ds[DS_SOLVER_ITERS];
   return ds[DS_SOLVER_ITERS];
 }
 

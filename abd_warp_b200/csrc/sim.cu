@@ -835,8 +835,6 @@ int abd_sim_create(const abd_scene_desc* d, const abd_params* prm, void* stream,
   ok(dalloc(&s.upper_ptr, n + 1));
   for (double** v : {&s.g, &s.dq}) ok(dalloc(v, 12 * (size_t)n));
   ok(dalloc(&s.kry_pub, 36 * (size_t)n));
-  ok(dalloc(&s.kry_spill, 72 * (size_t)n));
-  ok(cudaMalloc(&s.kry_pos, abd::krylov_pos_bytes(n)));
   if (ok(cudaMalloc(&s.cl_tab, abd::cluster_tables_bytes(n)))) {
     const abd::ClusterTables t = abd::cluster_tables_at(s.cl_tab, n);
     s.cl_ptr = t.cl_ptr;
@@ -946,7 +944,7 @@ int abd_sim_destroy(abd_sim* h) {
                   s.fixed, s.x, s.xk, s.body_box, s.pair_mask, s.row_ptr, s.upper_ptr, s.ij, s.adj_col,
                   s.adj_pair, s.pt_list, s.ee_list, s.vg_list, s.pair_cand, s.offdiag, s.pdiag, s.pgrad,
                   s.pair_active, s.pair_val, s.g, s.dq, s.diag,
-                  s.kry_pub, s.kry_spill, s.kry_pos, s.nb_act, s.partials, s.box, s.dpar, s.dint,
+                  s.kry_pub, s.kry_vec, s.kry_scal, s.kry_int, s.nb_act, s.partials, s.box, s.dpar, s.dint,
                   s.row_cnt, s.upper_cnt, s.nbr, s.fdof, s.chunk_box, s.vperm,
                   s.cl_tab, s.cl_inv, s.pair_wpre, s.act_pairs, s.chunk,
                   s.red_count, s.body_bnd, s.contacts, s.contacts_by_pair, s.ccd_cand, s.ecand, s.body_rest,
@@ -954,7 +952,7 @@ int abd_sim_destroy(abd_sim* h) {
                   s.chunk_act, s.fric, s.fric_mask, s.list, s.reg, s.ext, s.gh_q, s.x_ij, s.x_off, s.x_act, s.x_row, s.x_cnt};
   for (void* q : bufs)
     if (q) cudaFree(q);
-  for (abd::GraphSlot* g : {&s.g_ccd, &s.g_ccd_ev, &s.g_gh, &s.g_gh0, &s.g_ls, &s.g_ls_dev, &s.g_step})
+  for (abd::GraphSlot* g : {&s.g_ccd, &s.g_ccd_ev, &s.g_gh, &s.g_gh0, &s.g_ls, &s.g_ls_dev, &s.g_step, &s.g_solve, &s.g_solve_dq})
     if (g->exec) cudaGraphExecDestroy(g->exec);
   for (cudaStream_t q : {s.cap_stream, s.cap_stream2, s.cap_stream3, s.cap_stream4, s.cap_stream5, s.fork_a})
     if (q) cudaStreamDestroy(q);
@@ -1389,6 +1387,7 @@ int step_issue(abd_sim* h, const abd_states& st, double* x_view) {
         }))
       return q;
     s.loop.list = s.launches - l0;
+    s.loop.solve = 0;
     if (int q = abd::add_conditional(s.stream, hn, cudaGraphCondTypeWhile, &nbody)) return q;
     const long long l1 = s.launches;
     if (int q = abd::capture_body(s, nbody, s.cap_stream4, [&]() -> int {
@@ -1434,7 +1433,7 @@ int step_outcome(abd_sim* h, const abd::LoopLaunches& loop) {
   Sim& s = h->s;
   std::memcpy(s.hstat, s.hbox->dstat, sizeof(int) * abd::DS_NSLOTS);
   const abd::StepDev& S = s.hbox->step;
-  s.launches += (long long)S.it * loop.step + (long long)S.lists * loop.list;
+  s.launches += (long long)S.it * loop.step + (long long)S.lists * loop.list + (long long)S.lin * loop.solve;
   s.n_pairs = s.hstat[abd::DS_NPAIRS];
   s.n_adj = s.hstat[abd::DS_NADJ];
   const int bits = s.hstat[abd::DS_STATUS];
@@ -1551,7 +1550,7 @@ int joint_issue(abd_batch* b, const abd_states* st, double* const* x_view, std::
               }))
             return q;
           s.loop.list = s.launches - l0;
-          s.loop.step = 0;  // (an iteration has no kernels of its own)
+          s.loop.step = s.loop.solve = 0;  // (an iteration has no kernels of its own)
           b->loop[b->joint[k]] = s.loop;
           s.launches = l0;
           CK(cudaEventRecord(s.fork_ev[1], s.stream));
