@@ -39,7 +39,7 @@ namespace {
 
 inline unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-constexpr int kListShort = 1 << 16, kListLong = 1 << 18;  // candidates: the skin may grow below, shrinks above
+constexpr int kListShort = 1 << 15, kListLong = 1 << 18;  // candidates: the skin may grow below, shrinks above
 constexpr double kSkinMin = 1.0, kSkinMax = 64.0;         // in skin units (Sim::skin_unit)
 
 // The list's region around the step: its segment runs from the iterate q to q - dq when an
@@ -148,8 +148,7 @@ cudaError_t list_build(Sim& s, const abd_states& st) {
   cudaError_t e = list_pairs(s, fr ? s.fric_mask : nullptr);
   if (e == cudaSuccess) e = list_traverse(s);
   if (e != cudaSuccess) return e;
-  // (32 MB for a small scene's list and its line-search candidates)
-  const int very_long = (int)std::min((long long)INT_MAX, std::max(1LL << 20, 2 * ((long long)s.V + s.E)));
+  const int very_long = (int)std::min((long long)INT_MAX, std::max((long long)kListLong, ((long long)s.V + s.E) / 2));
   k_list_made<<<1, 1, 0, s.stream>>>(s.box, s.dint + kListBad, s.dpar, skin_unit(s, s.prm.dhat), s.cap_list, very_long,
                                      s.prof_on == 2 ? 1 : 0);
   ++s.launches;

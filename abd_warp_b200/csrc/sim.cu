@@ -203,7 +203,7 @@ int grow_list(Sim& s, int need) {
   ++s.cap_gen;  // every captured pass is keyed on it
   if (need < 0) return ABD_ERR_OVERFLOW;
   if (need > s.cap_list) {
-    const int cap = (int)std::min((long long)INT_MAX, std::max(need + need / 2LL, 2LL * s.cap_list));
+    const int cap = (int)std::min((long long)INT_MAX, std::max(s.cap_list ? 2LL * need : need, 2LL * s.cap_list));
     if (s.list) cudaFree(s.list);
     s.list = nullptr;
     s.cap_list = 0;  // (no memory: no capacity)
@@ -920,7 +920,9 @@ int abd_sim_create(const abd_scene_desc* d, const abd_params* prm, void* stream,
   if (!r) r = grow_fric(s, cap0(std::max(1024, 2 * n)));
   if (!r) r = grow_ccd(s, cap0(std::max(1 << 15, 32 * n)));
   if (!r) r = grow_ecand(s, cap0(std::max(1 << 15, 32 * n)));
-  if (!r) r = grow_list(s, cap0(std::max(1 << 15, 32 * n)));
+  // (a list that outgrows its capacity costs the step's rerun and a capture, in a batch of all its scenes)
+  const int list0 = (int)std::min(1LL << 18, std::max(1LL << 16, 24 * ((long long)V + E)));
+  if (!r) r = grow_list(s, cap0(std::max(32 * n, list0)));
   s.cap_pt = 0;
   s.cap_ee = 0;
   if (!r) r = grow_lists(s, cap0(std::max(1 << 14, V / 4)), cap0(std::max(1 << 14, E / 4)));
