@@ -496,7 +496,8 @@ constexpr int kParK = 4;          // dpar slot of a batch's trial count
 constexpr int kParAlpha = 5;      // dpar slots of its step lengths
 constexpr int kParSkin = kParAlpha + kLsMax;  // dpar slot of the kept list's displacement: what it was made with
 constexpr int kParSkinNext = kParSkin + 1;    // and of the next list's
-constexpr int kNPar = kParSkinNext + 1;
+constexpr int kParSkinMost = kParSkinNext + 1;  // the largest it may grow to
+constexpr int kNPar = kParSkinMost + 1;
 
 // dstat layout
 enum : int {

@@ -17,13 +17,20 @@
 // steps are long, make it every fourth iteration.
 //
 // The skin follows the scene (from list to list: the DOFs are checked against the one that the list in
-// use was made with): it doubles when an iteration leaves the region that the same step
-// made, while the list is short (a pass over 65k candidates takes about as long as one over 10k: a
-// thread each on 296 CTAs), and halves when the list is long (several candidates a thread; the next step
-// then makes the list again).  A list that is very long for its scene is not given the memory: the step
-// starts again with half the skin, down to the least one.  The skin is counted in units of dhat, or of
-// 1/64 of the bodies' half extent where that is less: with dhat in place of it, 28 bodies of 0.2 m with
-// dhat = 60 mm made lists of 20 GB and took 340 ms a step (2.2 ms without a list).
+// use was made with).  It doubles when a step's iteration asks for a list while the list is short: the
+// next one is four to five times as long, which the GPU still takes in a round or two, a candidate a
+// thread (a pass over 65k candidates takes about as long as one over 10k).  It halves when the list is
+// long, and the next step makes the list again.  A list that outgrows its capacity and is long for its
+// scene is not given the memory: the step starts again with half the skin, the most it may have from
+// then on (else the rerun would double it as the run did), down to the least, and only then with a larger
+// list.  With 65k and 262k candidates as the bounds the list of 16 spheres alternated between the two, and
+// where many scenes share the GPU long lists cost as much as they are long: 48 scenes of four spheres
+// with 2,562 vertices took 24.1 ms a step, 22.0 with these bounds, 21.4 without a list (16 spheres,
+// ten steps and back: 88 and 80 ms).
+//
+// The skin is counted in units of dhat, or of 1/64 of the bodies' half extent where that is less: with
+// dhat in place of it, 28 bodies of 0.2 m with dhat = 60 mm made lists of 20 GB and took 340 ms a step
+// (2.2 ms without a list; 1.3 now).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,8 +46,8 @@ namespace {
 
 inline unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-constexpr int kListShort = 1 << 15, kListLong = 1 << 18;  // candidates: the skin may grow below, shrinks above
-constexpr double kSkinMin = 1.0, kSkinMax = 64.0;         // in skin units (Sim::skin_unit)
+constexpr int kListShort = 1 << 14, kListLong = 1 << 17;  // candidates: the skin may grow below, shrinks above
+constexpr double kSkinMin = 1.0;                          // in skin units (skin_unit)
 
 // The list's region around the step: its segment runs from the iterate q to q - dq when an
 // iteration asked for the list (its solve is done), else, at the step's start, to the prediction
@@ -108,7 +115,8 @@ __global__ void k_list_made(Mailbox* box, int* bad, double* dpar, double unit, i
   if (box->dstat[DS_STATUS] & kRerunMask) {
     if ((box->dstat[DS_STATUS] & ST_LIST_OVERFLOW) && (unsigned)box->dstat[DS_NLIST] > (unsigned)very_long &&
         skin > kSkinMin * unit) {
-      dpar[kParSkinNext] = fmax(0.5 * skin, kSkinMin * unit);
+      // (for good: a rerun that doubled its displacement again would end where this one did)
+      dpar[kParSkinNext] = dpar[kParSkinMost] = fmax(0.5 * skin, kSkinMin * unit);
       S.shrunk = 1;  // (the host does not grow the list)
     }
     return;
@@ -117,7 +125,7 @@ __global__ void k_list_made(Mailbox* box, int* bad, double* dpar, double unit, i
   ++S.lists;
   const int m = min(box->dstat[DS_NLIST], cap_list);
   dpar[kParSkin] = skin;
-  if (S.resume && m <= kListShort) dpar[kParSkinNext] = fmin(2.0 * skin, kSkinMax * unit);
+  if (S.resume && m <= kListShort) dpar[kParSkinNext] = fmin(2.0 * skin, dpar[kParSkinMost]);
   else if (m > kListLong) dpar[kParSkinNext] = fmax(0.5 * skin, kSkinMin * unit);
 }
 

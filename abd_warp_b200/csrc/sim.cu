@@ -290,7 +290,8 @@ int sync_read(Sim& s) {
 
 constexpr int kRerun = -1;
 
-constexpr double kSkin0 = 8.0;  // first skin of the kept candidate list, in its units (listpass.cu adapts it)
+constexpr double kSkin0 = 8.0, kSkinMost = 64.0;  // first and largest skin of the kept candidate list, in its
+                                                  // units (listpass.cu adapts it)
 
 // After sync_read: grow every capacity whose overflow bit is set and clear those bits.
 // Returns kRerun when the pass has to be rerun, 0 when it is complete, or an ABD error.
@@ -900,6 +901,7 @@ int abd_sim_create(const abd_scene_desc* d, const abd_params* prm, void* stream,
     for (int k = 0; k < abd::kNPar; ++k) s.hpar[k] = 0.0;
     s.hpar[1] = 1.0;
     s.hpar[abd::kParSkinNext] = kSkin0 * abd::skin_unit(s, prm->dhat);
+    s.hpar[abd::kParSkinMost] = kSkinMost * abd::skin_unit(s, prm->dhat);
     e = cudaMemcpyAsync(s.dpar, s.hpar, abd::kNPar * sizeof(double), cudaMemcpyHostToDevice, s.stream);
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(s.red_count, 0, sizeof(int) * abd::kRedSlots, s.stream);
@@ -979,7 +981,9 @@ int abd_sim_set_params(abd_sim* h, const abd_params* prm) {
   // the kept list belongs to the old parameters; its skin starts again
   CK(cudaMemsetAsync(h->s.dint + abd::kListBad, 1, sizeof(int), h->s.stream));
   h->s.hpar[abd::kParSkinNext] = kSkin0 * abd::skin_unit(h->s, prm->dhat);
-  CK(cudaMemcpyAsync(h->s.dpar + abd::kParSkinNext, h->s.hpar + abd::kParSkinNext, sizeof(double),
+  h->s.hpar[abd::kParSkinMost] = kSkinMost * abd::skin_unit(h->s, prm->dhat);
+  static_assert(abd::kParSkinMost == abd::kParSkinNext + 1, "copied together");
+  CK(cudaMemcpyAsync(h->s.dpar + abd::kParSkinNext, h->s.hpar + abd::kParSkinNext, 2 * sizeof(double),
                      cudaMemcpyHostToDevice, h->s.stream));
   h->s.prm = *prm;
   ++h->s.prm_version;  // parameters are kernel arguments of the captured passes
