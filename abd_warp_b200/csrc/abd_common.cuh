@@ -698,7 +698,7 @@ cudaError_t round_end(Sim& s, cudaGraphConditionalHandle h_round);
 cudaError_t newton_end(Sim& s, const abd_states& st, cudaGraphConditionalHandle h);
 // newton_batch.cu: the Newton iterations of many small scenes in one kernel, a cluster of CTAs each
 constexpr int kBatchLeast = 9;   // fewer scenes step as branches of their own
-bool batch_loop_takes(const Sim& s);
+bool batch_loop_takes(const Sim& s, int scenes);   // (of the batch)
 int batch_loop_ctas(const Sim& s, int scenes);     // CTAs of a scene's cluster
 size_t batch_loop_bytes();                         // a scene's arguments, in device memory
 void batch_loop_args(Sim& s, const abd_states& st, int C, void* host);

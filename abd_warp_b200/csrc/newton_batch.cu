@@ -9,11 +9,14 @@
 // immaterial, so the results are the kernels', bit for bit.
 //
 // The rule (batch_loop_takes): scenes with the reference's contact model, no friction and the CG
-// solver, of at most kLoopBodies bodies and kLoopPrims vertices and edges, when the batch has
-// kBatchLeast of them.  A larger scene's phases want more SMs than a cluster has; fewer scenes have a
-// queue each, and an iteration by kernels over the whole GPU takes 60 to 75 us where a cluster
-// takes 75 (16 CTAs) to 140 us (4).  Five steps of 48 scenes of 2 to 48 bodies: 52 to 60 ms as
-// branches, 21 to 27 ms so.
+// solver, when the batch has kBatchLeast of them; a scene of at most kLoopBodies bodies, and of vertices
+// and edges at most kLoopPrims or, if that is more, kLoopShare for each scene of the batch.  A larger
+// scene's phases want more SMs than a cluster has, and get them while few scenes share the GPU; with
+// fewer scenes than the eight queues each has one.  Measured, a step as branches -> in this kernel:
+//   scenes   9 of 4 to 14 bodies 2.5 -> 1.7 ms, 48 11.6 -> 4.0, 512 198 -> 28 (6: 1.9 -> 1.5, 4: 1.3 -> 1.4);
+//   bodies   12 scenes of 127 3.9 -> 2.6 ms, of 176 3.9 -> 3.1;
+//   vertices and edges a scene   41,000: 9 scenes 4.2 -> 3.6 ms, 48 21.5 -> 13.5;  82,000: 9 scenes
+//            5.3 -> 6.7, 24 11.3 -> 9.9;  164,000: 12 scenes 9.8 -> 13.6, 24 18.2 -> 18.1, 48 36.6 -> 32.9.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,7 +39,7 @@ namespace cg = cooperative_groups;
 
 constexpr int LT = assemble::PT_THREADS;  // threads of a CTA
 constexpr int kLoopCtas = 16;             // most CTAs of a cluster
-constexpr int kLoopBodies = 64, kLoopPrims = 1 << 15;
+constexpr int kLoopBodies = 192, kLoopPrims = 1 << 16, kLoopShare = 1 << 12;
 constexpr int kLoopSlots = 2 * 148;       // CTAs resident at a time: two per SM (128 registers)
 static_assert(LT >= 160, "a body's pass");
 // four CTAs at least, so that a preconditioner cluster's panels fit (abd_precond.cuh)
@@ -312,9 +315,9 @@ cudaError_t prepare_newton_batch(Sim& s) {
   return cudaSuccess;
 }
 
-bool batch_loop_takes(const Sim& s) {
+bool batch_loop_takes(const Sim& s, int scenes) {
   return s.prm.solver == 1 && !s.prm.ipc_full && !(s.prm.friction_mu > 0.0) && s.max_loop_ctas > 0 &&
-         s.n <= kLoopBodies && s.V + s.E <= kLoopPrims;
+         s.n <= kLoopBodies && (long long)s.V + s.E <= std::max((long long)kLoopPrims, (long long)kLoopShare * scenes);
 }
 
 // As many CTAs for a scene as make up to twice what the GPU holds at a time: the largest scenes come

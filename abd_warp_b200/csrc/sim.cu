@@ -1707,7 +1707,7 @@ int abd_batch_step(abd_batch* b, const abd_states* st, double* const* x_view, ab
     // the small scenes' Newton iterations share a kernel when there are enough of them
     b->joint.clear();
     for (int i = 0; i < n; ++i)
-      if (abd::batch_loop_takes(b->sims[i]->s)) b->joint.push_back(i);
+      if (abd::batch_loop_takes(b->sims[i]->s, n)) b->joint.push_back(i);
     if ((int)b->joint.size() < abd::kBatchLeast) b->joint.clear();
     // the largest first: the launch ends with its longest scenes
     std::stable_sort(b->joint.begin(), b->joint.end(), [&](int i, int j) {
