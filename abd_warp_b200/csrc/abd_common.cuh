@@ -497,7 +497,8 @@ constexpr int kParAlpha = 5;      // dpar slots of its step lengths
 constexpr int kParSkin = kParAlpha + kLsMax;  // dpar slot of the kept list's displacement: what it was made with
 constexpr int kParSkinNext = kParSkin + 1;    // and of the next list's
 constexpr int kParSkinMost = kParSkinNext + 1;  // the largest it may grow to
-constexpr int kNPar = kParSkinMost + 1;
+constexpr int kParListNeed = kParSkinMost + 1;  // candidates of the last list, when it outgrew its capacity
+constexpr int kNPar = kParListNeed + 1;
 
 // dstat layout
 enum : int {

@@ -113,8 +113,11 @@ __global__ void k_list_made(Mailbox* box, int* bad, double* dpar, double unit, i
   S.t0 = ~0ULL;
   S.t1 = 0ULL;
   if (box->dstat[DS_STATUS] & kRerunMask) {
-    if ((box->dstat[DS_STATUS] & ST_LIST_OVERFLOW) && (unsigned)box->dstat[DS_NLIST] > (unsigned)very_long &&
-        skin > kSkinMin * unit) {
+    const double need = (double)(unsigned)box->dstat[DS_NLIST], last = dpar[kParListNeed];
+    if (!(box->dstat[DS_STATUS] & ST_LIST_OVERFLOW)) return;
+    dpar[kParListNeed] = need;
+    // (a list that half the skin left as long is long for the segment's sake)
+    if (need > (double)very_long && skin > kSkinMin * unit && !(last > 0.0 && need > 0.75 * last)) {
       // (for good: a rerun that doubled its displacement again would end where this one did)
       dpar[kParSkinNext] = dpar[kParSkinMost] = fmax(0.5 * skin, kSkinMin * unit);
       S.shrunk = 1;  // (the host does not grow the list)
@@ -122,6 +125,7 @@ __global__ void k_list_made(Mailbox* box, int* bad, double* dpar, double unit, i
     return;
   }
   *bad = 0;
+  dpar[kParListNeed] = 0.0;
   ++S.lists;
   const int m = min(box->dstat[DS_NLIST], cap_list);
   dpar[kParSkin] = skin;
