@@ -351,13 +351,12 @@ struct Sim {
   GraphSlot g_solve, g_solve_dq;   // large solves (of adj_x, of dq)
   double* adj_x = nullptr;         // [12 n] the adjoint solve's unknown lambda
   cudaStream_t cap_stream3 = nullptr, cap_stream4 = nullptr;  // capture the loop's bodies
-  // side branches of a pass (the GH pass's clustering, the host loop's dot products): a stream
-  // joins the capture it forks from until that capture ends, so the device loop's Newton body
-  // has its own (fork_a); null: cap_stream2
-  cudaStream_t fork_a = nullptr, side = nullptr;
+  // side branch of the device loop's Newton body (the clustering): a stream joins the capture it
+  // forks from until that capture ends, so cap_stream2 is not free there
+  cudaStream_t fork_a = nullptr;
   // A device-loop step (in_device_loop: its capture is in progress) makes its candidate list in
   // an IF node
-  cudaStream_t cap_stream5 = nullptr;  // captures that IF node's body
+  cudaStream_t cap_stream5 = nullptr;  // captures that IF node's body, and a large solve's loop
   bool in_device_loop = false;
   double* dq_save = nullptr;       // [12 n] dq at the start of a device-loop step (for a rerun)
   LoopLaunches loop;               // of the step that is being captured
@@ -401,7 +400,6 @@ struct Sim {
   int cap_ecand = 0;
   int4* ecand = nullptr;
   int list_counts[4] = {0, 0, 0, 0};  // pairs, PT, EE, VG of the last list culling
-  double* pair_val = nullptr;      // [cap_pairs] energy or toi per pair
 
 
   // Newton system
@@ -430,7 +428,6 @@ struct Sim {
   int* red_count = nullptr;        // [kRedSlots] CTAs done per reduction (last CTA finishes)
   int* dstat = nullptr;            // = box->dstat: [0] status, [1..] counters
   int* hstat = nullptr;            // pinned: [0, 16) mirror of dstat, [16, 32) host scratch
-  double* hval = nullptr;          // pinned host scalars
   unsigned long long* dmin = nullptr;  // = &box->toi_key
 };
 

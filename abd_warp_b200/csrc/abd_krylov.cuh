@@ -29,7 +29,6 @@ struct KrylovArgs {
   int n, maxit;
   const double *diag, *offdiag, *g;
   const int *row_ptr, *adj_col, *adj_pair, *pair_active, *fixed;
-  const int2* ij;
   int2* nb;                 // [adjacency capacity] active neighbours per row: (body, 2 pair + side)
   const int *cl_ptr, *cl_body, *body_cl;
   const long long* cl_off;

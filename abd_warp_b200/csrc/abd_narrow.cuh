@@ -71,7 +71,7 @@ struct NarrowArgs {
   int cap_pt, cap_ee;
   int* pair_cand;
   int* dstat;
-  double *offdiag, *pdiag, *pgrad, *pair_val;
+  double *offdiag, *pdiag, *pgrad;
   int* pair_active;
 };
 

@@ -16,7 +16,6 @@ constexpr int BP = 3;  // most bodies of a preconditioner cluster that one CTA i
 struct SolverArgs {
   const double *diag, *offdiag;
   const int *row_ptr, *adj_col, *adj_pair, *pair_active, *fixed;
-  const int2* ij;
   const int* ncl_dev; // clusters (formed on the device)
   const int* dstat;
   const int* resume;  // device loop: set when the iteration's solve is done (or null)

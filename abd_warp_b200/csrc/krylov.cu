@@ -50,7 +50,6 @@ KrylovArgs krylov_args(Sim& s, double* x, bool tally, int C, size_t* smem_out) {
   a.adj_pair = s.adj_pair;
   a.pair_active = s.pair_active;
   a.fixed = s.fixed;
-  a.ij = s.ij;
   a.nb = s.nb_act;
   a.cl_ptr = s.cl_ptr;
   a.cl_body = s.cl_body;

@@ -107,7 +107,6 @@ NarrowArgs narrow_args(Sim& s, int mode, const double* A, const double* p, const
   a.offdiag = s.offdiag;
   a.pdiag = s.pdiag;
   a.pgrad = s.pgrad;
-  a.pair_val = s.pair_val;
   a.pair_active = s.pair_active;
   return a;
 }

@@ -140,14 +140,14 @@ int grow_pairs(Sim& s, int need) {
   const int cap = std::max(need + need / 2, 2 * s.cap_pairs);
   const int cap_adj = 2 * cap;
   for (void* q : {(void*)s.ij, (void*)s.adj_col, (void*)s.adj_pair, (void*)s.pair_cand, (void*)s.offdiag,
-                  (void*)s.pdiag, (void*)s.pgrad, (void*)s.pair_active, (void*)s.pair_val, (void*)s.nb_act})
+                  (void*)s.pdiag, (void*)s.pgrad, (void*)s.pair_active, (void*)s.nb_act})
     if (q) cudaFree(q);
   s.cap_pairs = cap;
   s.cap_adj = cap_adj;
   if (dalloc(&s.ij, cap) || dalloc(&s.adj_col, cap_adj) || dalloc(&s.adj_pair, cap_adj) ||
       dalloc(&s.pair_cand, 4 * (size_t)cap) || dalloc(&s.offdiag, 288 * (size_t)cap) ||
       dalloc(&s.pdiag, 288 * (size_t)cap) || dalloc(&s.pgrad, 24 * (size_t)cap) || dalloc(&s.pair_active, cap) ||
-      dalloc(&s.pair_val, cap) || dalloc(&s.nb_act, cap_adj))
+      dalloc(&s.nb_act, cap_adj))
     return ABD_ERR_OVERFLOW;
   // zeroed so that the body ids of a pass that overflowed are still valid indices
   if (cudaMemsetAsync(s.ij, 0, sizeof(int2) * cap, s.stream) ||
@@ -516,7 +516,7 @@ int gh_issue(abd_sim* h, const abd_states& st, const double* A, const double* p,
   CK(abd::gh_superset_check(s, &st, sup_mode));
   int r = culling(h, &d, nullptr, s.x, nullptr, abd::NARROW_GH);
   if (r) return r;
-  const cudaStream_t side = s.side ? s.side : s.cap_stream2;
+  const cudaStream_t side = s.cap_stream2;
   CK(cudaEventRecord(s.fork_ev[0], s.stream));
   CK(cudaStreamWaitEvent(side, s.fork_ev[0], 0));
   CK(abd::cluster_tables(s, side));
@@ -885,7 +885,6 @@ int abd_sim_create(const abd_scene_desc* d, const abd_params* prm, void* stream,
   if (e == cudaSuccess) e = cudaHostAlloc((void**)&s.hstat, 32 * sizeof(int), cudaHostAllocDefault);
   if (e == cudaSuccess) e = cudaHostAlloc((void**)&s.hbox, sizeof(abd::Mailbox), cudaHostAllocDefault);
   if (e == cudaSuccess) e = cudaHostAlloc((void**)&s.hpar, abd::kNPar * sizeof(double), cudaHostAllocDefault);
-  if (e == cudaSuccess) e = cudaHostAlloc((void**)&s.hval, 32 * sizeof(double), cudaHostAllocDefault);
   if (e == cudaSuccess) e = abd::rest_boxes(s);
   if (e == cudaSuccess && abd::prepare_solver(s) != ABD_OK) e = cudaErrorUnknown;
   if (e == cudaSuccess) e = abd::prepare_krylov(s);
@@ -947,7 +946,7 @@ int abd_sim_destroy(abd_sim* h) {
   void* bufs[] = {s.voff, s.toff, s.eoff, s.vbody, s.tbody, s.ebody, s.tris, s.edges, s.x0, s.mass, s.I0,
                   s.fixed, s.x, s.xk, s.body_box, s.pair_mask, s.row_ptr, s.upper_ptr, s.ij, s.adj_col,
                   s.adj_pair, s.pt_list, s.ee_list, s.vg_list, s.pair_cand, s.offdiag, s.pdiag, s.pgrad,
-                  s.pair_active, s.pair_val, s.g, s.dq, s.diag,
+                  s.pair_active, s.g, s.dq, s.diag,
                   s.kry_pub, s.kry_vec, s.kry_scal, s.kry_int, s.nb_act, s.partials, s.box, s.dpar, s.dint,
                   s.row_cnt, s.upper_cnt, s.nbr, s.fdof, s.chunk_box, s.vperm,
                   s.cl_tab, s.cl_inv, s.pair_wpre, s.act_pairs, s.chunk,
@@ -962,7 +961,7 @@ int abd_sim_destroy(abd_sim* h) {
     if (q) cudaStreamDestroy(q);
   for (cudaEvent_t ev : {s.prof_ev[0], s.prof_ev[1], s.fork_ev[0], s.fork_ev[1], s.fork_ev[2], s.fork_ev[3]})
     if (ev) cudaEventDestroy(ev);
-  for (void* q : {(void*)s.hstat, (void*)s.hval, (void*)s.hbox, (void*)s.hpar})
+  for (void* q : {(void*)s.hstat, (void*)s.hbox, (void*)s.hpar})
     if (q) cudaFreeHost(q);
   delete h;
   return ABD_OK;

@@ -27,7 +27,6 @@ SolverArgs solver_args(Sim& s) {
   a.adj_pair = s.adj_pair;
   a.pair_active = s.pair_active;
   a.fixed = s.fixed;
-  a.ij = s.ij;
   a.ncl_dev = s.ncl_dev;
   a.dstat = s.dstat;
   a.resume = s.in_device_loop ? &s.box->step.resume : nullptr;
