@@ -1,10 +1,10 @@
 """Batched scenes: many independent scenes stepped together (``abd_batch_*`` in the C ABI).
 
 The reference steps one scene per ``AffineBodySimulator``.  :class:`BatchSimulator` holds one
-simulator per scene and steps them all with one CUDA graph launch: each scene's step (its
-Newton iterations as a device loop) is a branch of the graph, so the scenes' iterations run
-concurrently on the GPU while each keeps its own iteration counts, line search and
-convergence -- every scene's result is the one its own ``step()`` gives.
+simulator per scene and steps them all with one CUDA graph launch.  The Newton iterations of nine
+or more small scenes share one kernel of the graph (a cluster of thread blocks per scene); every other
+scene's step is a branch of its own.  Each scene keeps its own iteration counts, line search and
+convergence -- its result is the one its own ``step()`` gives.
 """
 from __future__ import annotations
 

@@ -27,8 +27,8 @@ struct abd_sim {
   abd::Sim s;
 };
 
-// Independent scenes stepped together: one CUDA graph holds every scene's device-loop step as
-// a branch of its own (see abd_batch_step)
+// Independent scenes stepped together by one CUDA graph: many small scenes with their Newton iterations in
+// one kernel (joint), every other scene's device-loop step as a branch of its own (see abd_batch_step)
 struct abd_batch {
   std::vector<abd_sim*> sims;
   cudaStream_t stream = nullptr;      // the stream the steps are launched on

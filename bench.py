@@ -16,8 +16,8 @@ value: steps/s on device-resident states.  e2e: the same steps through the publi
 host buffers: every step copies its inputs (A0, p0, Adot, pdot) in from pinned host memory,
 and copies the new vertex positions and the new states back, inside the timed region.
 
-roofline: the narrow-phase kernel of the CCD pass, which also collects the line-search
-candidates (the largest share of the step).  The step runs as one CUDA graph whose Newton loop
+roofline: the narrow-phase tree traversal, which makes the step's kept candidate list (in the host
+loop: the CCD pass's, which also collects the line-search candidates).  The step runs as one CUDA graph whose Newton loop
 is a device-side WHILE node, where events cannot be recorded, so every launch of the kernel
 inside the timed region is timed by the GPU's global timer: the kernel records the start of
 its first CTA and the end of its last, on the stream it runs on.  The data it moves
@@ -503,8 +503,8 @@ def main():
         "e2e": {"value": e2e_value, "unit": "steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "gpu_launches": int(launches),
         "clocks": clk,
-        "roofline": {"kernel": "k_chunk_narrow<CCD_LS> (narrow phase of the CCD pass, which also collects "
-                               "the line-search candidates)", "bound": "hbm",
+        "roofline": {"kernel": "k_chunk_narrow<CCD_LS> (the narrow phase's tree traversal, which makes the "
+                               "step's kept candidate list)", "bound": "hbm",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": bytes_per_launch * NARROW_DRAM_PER_ALG_BYTE,

@@ -143,11 +143,11 @@ int abd_step(abd_sim* sim, const abd_states* st, double* x_view_dev, abd_step_in
  * destroys them after the batch); stream is where the batch's steps run (NULL: legacy default
  * stream).  abd_batch_step steps every scene once: st[i] are scene i's states, x_view[i] its
  * vertex positions out (x_view or any x_view[i] may be NULL), info[i] its step info (info may
- * be NULL).  All scenes' device-loop steps are one CUDA graph, each scene a branch of its own
- * that holds its Newton loop, so one launch runs every scene's iterations concurrently with
- * each scene's own iteration counts, line search and convergence: each scene's result is the
- * one abd_step gives it.  A scene whose list overflowed is stepped again alone after the
- * list grew.  Needs alpha_min > 2^-15 in every scene (else ABD_ERR_INVALID).  Returns the
+ * be NULL).  All scenes' steps are one CUDA graph: the Newton iterations of nine or more small
+ * scenes share a kernel, every other scene is a branch of its own that holds its Newton loop.  Each
+ * scene has its own iteration counts, line search and convergence: its result is the one
+ * abd_step gives it.  A scene whose list overflowed is stepped again alone after the list
+ * grew.  Needs alpha_min > 2^-15 in every scene (else ABD_ERR_INVALID).  Returns the
  * first error of a scene, or ABD_OK. */
 int abd_batch_create(int n, abd_sim* const* sims, void* stream, abd_batch** out);
 int abd_batch_destroy(abd_batch* batch);
