@@ -494,6 +494,7 @@ constexpr int kParAlpha = 5;      // dpar slots of its step lengths
 constexpr int kParSkin = kParAlpha + kLsMax;  // dpar slot of the kept list's displacement: what it was made with
 constexpr int kParSkinNext = kParSkin + 1;    // and of the next list's
 constexpr int kParSkinMost = kParSkinNext + 1;  // the largest it may grow to
+constexpr int kListShort = 1 << 14, kListLong = 1 << 17;  // candidates: it may grow below, shrinks above (listpass.cu)
 constexpr int kParListNeed = kParSkinMost + 1;  // candidates of the last list, when it outgrew its capacity
 constexpr int kNPar = kParListNeed + 1;
 

@@ -71,15 +71,18 @@ __global__ void k_step_begin(Mailbox* box, cudaGraphConditionalHandle h, int n, 
   cudaGraphSetConditional(h, 1u);
 }
 
-// A round's start: the kept list is made when it has to be, then Newton iterations run.
+// A round's start: the kept list is made when it has to be (for an iteration that left the region of a
+// short one, with twice the displacement: listpass.cu), then Newton iterations run.
 // shared: the scene's iterations are in its batch's kernel (newton_batch.cu), if it still runs.
-__global__ void k_round_begin(Mailbox* box, const int* bad, int* cand, int cap_pairs, cudaGraphConditionalHandle h_list,
-                              cudaGraphConditionalHandle h_newton, int shared) {
+__global__ void k_round_begin(Mailbox* box, const int* bad, double* dpar, int* cand, int cap_pairs,
+                              cudaGraphConditionalHandle h_list, cudaGraphConditionalHandle h_newton, int shared) {
   int* const ds = box->dstat;
   const bool run = !shared || box->step.run;
   if (threadIdx.x == 0) {
     box->step.again = 0;
     if (run) ++box->step.rounds;
+    if (run && *bad && box->step.resume && ds[DS_NLIST] <= kListShort)
+      dpar[kParSkinNext] = fmin(2.0 * dpar[kParSkinNext], dpar[kParSkinMost]);
     cudaGraphSetConditional(h_list, run && *bad ? 1u : 0u);
     if (!shared) cudaGraphSetConditional(h_newton, 1u);
   }
@@ -211,8 +214,8 @@ cudaError_t step_begin(Sim& s, const abd_states& st, cudaGraphConditionalHandle 
 }
 
 cudaError_t round_begin(Sim& s, cudaGraphConditionalHandle h_list, cudaGraphConditionalHandle h_newton, bool shared) {
-  k_round_begin<<<1, shared ? 128 : 1024, 0, s.stream>>>(s.box, s.dint + kListBad, s.pair_cand, s.cap_pairs, h_list,
-                                                        h_newton, shared ? 1 : 0);
+  k_round_begin<<<1, shared ? 128 : 1024, 0, s.stream>>>(s.box, s.dint + kListBad, s.dpar, s.pair_cand, s.cap_pairs,
+                                                        h_list, h_newton, shared ? 1 : 0);
   ++s.launches;
   return cudaGetLastError();
 }

@@ -920,7 +920,6 @@ int abd_sim_create(const abd_scene_desc* d, const abd_params* prm, void* stream,
   if (!r) r = grow_contacts(s, cap0(std::max(4096, 8 * n)));
   if (!r) r = grow_fric(s, cap0(std::max(1024, 2 * n)));
   if (!r) r = grow_ccd(s, cap0(std::max(1 << 15, 32 * n)));
-  if (!r) r = grow_ecand(s, cap0(std::max(1 << 15, 32 * n)));
   // (a list that outgrows its capacity costs the step's rerun and a capture, in a batch of all its scenes)
   const int list0 = (int)std::min(1LL << 18, std::max(1LL << 16, 24 * ((long long)V + E)));
   if (!r) r = grow_list(s, cap0(std::max(32 * n, list0)));
