@@ -20,16 +20,15 @@
 // use was made with).  It doubles when a step's iteration asks for a list while the list is short
 // (k_round_begin): the new one is four to five times as long, which the GPU still takes in a round or
 // two, a candidate a thread (a pass over 65k candidates takes about as long as one over 10k).  (Doubled
-// only for the list after that, the same step often asked again: 512 scenes stepped together went through
-// a third round, 20.0 ms a step against 19.3, and 16 spheres' ten steps and back took 91 ms against 87.)
-// It halves when the list is
-// long, and the next step makes the list again.  A list that outgrows its capacity and is long for its
-// scene is not given the memory: the step starts again with half the skin, the most it may have from
-// then on (else the rerun would double it as the run did), down to the least, and only then with a larger
-// list.  With 65k and 262k candidates as the bounds the list of 16 spheres alternated between the two, and
-// where many scenes share the GPU long lists cost as much as they are long: 48 scenes of four spheres
-// with 2,562 vertices took 24.1 ms a step, 22.0 with these bounds, 21.4 without a list (16 spheres,
-// ten steps and back: 88 and 80 ms).
+// only for the list after that, the same step often asked again: 512 scenes stepped together went
+// through a third round, 20.0 ms a step against 19.3, and 16 spheres' ten steps and back took 91 ms
+// against 87.)  It halves when the list is long, and the next step makes the list again.  A list that
+// outgrows its capacity and is long for its scene is not given the memory: the step starts again with
+// half the skin, the most it may have from then on (else the rerun would double it as the run did),
+// down to the least; only a list that this does not shorten gets a larger buffer.  With 65k and 262k
+// candidates as the bounds the list of 16 spheres alternated between the two, and where many scenes
+// share the GPU long lists cost as much as they are long: 48 scenes of four spheres with 2,562
+// vertices took 24.1 ms a step, 22.0 with these bounds, 21.4 without a list.
 //
 // The skin is counted in units of dhat, or of 1/64 of the bodies' half extent where that is less: with
 // dhat in place of it, 28 bodies of 0.2 m with dhat = 60 mm made lists of 20 GB and took 340 ms a step
